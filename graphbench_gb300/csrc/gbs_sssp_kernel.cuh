@@ -421,6 +421,45 @@ __device__ __forceinline__ void cand_drain(const SsspArgs &a, const Targets &t, 
     else if (nc) cand_flush<WT, 1>(a, t, nc, nc, imp, loc);
 }
 
+// One round of relax_group: edges [k0, k0 + 32 U) of the warp's rows, U per lane
+// (lane l's row holds edges [excl, ..) of them).
+template <int WT, int U>
+__device__ __forceinline__ void relax_round(const SsspArgs &a, const Targets &t, uint32_t u,
+                                            typename Arith<WT>::D du, uint32_t s, uint32_t excl, uint32_t total,
+                                            uint32_t k0, uint32_t &nc, uint32_t &imp, Local &loc) {
+    const unsigned FULL = 0xffffffffu;
+    const unsigned lane = lane_id();
+    uint32_t v[U], uo[U];
+    typename Arith<WT>::Wt w[U];
+    typename Arith<WT>::D duo[U];
+    bool val[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const uint32_t k = k0 + 32u * j + lane;
+        int owner = 0;
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+            const int cand = owner + step;
+            const uint32_t ex = __shfl_sync(FULL, excl, cand);
+            if (ex <= k) owner = cand;
+        }
+        const uint32_t so = __shfl_sync(FULL, s, owner);
+        const uint32_t exo = __shfl_sync(FULL, excl, owner);
+        uo[j] = __shfl_sync(FULL, u, owner);
+        duo[j] = __shfl_sync(FULL, du, owner);
+        val[j] = k < total;
+        v[j] = 0;
+        w[j] = 0;
+        if (val[j]) {
+            const uint32_t e = so + (k - exo);
+            const uint2 ew = ld_stream(a.g.adj + e);
+            v[j] = ew.x;
+            w[j] = weight_at<WT>(a, e, ew);
+        }
+    }
+    relax_candidates<WT>(a, t, val, v, w, uo, duo, nc, imp, loc);
+}
+
 // Warp-collective: relaxes edges [s, s+len) of source u (distance bits du)
 // given by every lane (len may be 0), kUnroll x 32 edges per round.
 template <int WT>
@@ -437,38 +476,12 @@ __device__ __forceinline__ void relax_group(const SsspArgs &a, const Targets &t,
     }
     const uint32_t total = __shfl_sync(FULL, incl, 31);
     const uint32_t excl = incl - len;
-    for (uint32_t k0 = 0; k0 < total; k0 += 32u * kUnroll) {
-        uint32_t v[kUnroll], uo[kUnroll];
-        typename Arith<WT>::Wt w[kUnroll];
-        typename Arith<WT>::D duo[kUnroll];
-        bool val[kUnroll];
-#pragma unroll
-        for (int j = 0; j < kUnroll; ++j) {
-            const uint32_t k = k0 + 32u * j + lane;
-            int owner = 0;
-#pragma unroll
-            for (int step = 16; step >= 1; step >>= 1) {
-                const int cand = owner + step;
-                const uint32_t ex = __shfl_sync(FULL, excl, cand);
-                if (ex <= k) owner = cand;
-            }
-            const uint32_t so = __shfl_sync(FULL, s, owner);
-            const uint32_t exo = __shfl_sync(FULL, excl, owner);
-            uo[j] = __shfl_sync(FULL, u, owner);
-            duo[j] = __shfl_sync(FULL, du, owner);
-            val[j] = k < total;
-            v[j] = 0;
-            w[j] = 0;
-            if (val[j]) {
-                const uint32_t e = so + (k - exo);
-                const uint2 ew = ld_stream(a.g.adj + e);
-                v[j] = ew.x;
-                w[j] = weight_at<WT>(a, e, ew);
-            }
-        }
-        relax_candidates<WT>(a, t, val, v, w, uo, duo, nc, imp, loc);
-    }
+    // the last 32 edges or fewer take one round of one edge per lane: a scan of
+    // a few short rows (a grid's) would run the owner search of 128 slots for them
+    uint32_t k0 = 0;
+    for (; k0 + 32u < total; k0 += 32u * kUnroll)
+        relax_round<WT, kUnroll>(a, t, u, du, s, excl, total, k0, nc, imp, loc);
+    if (k0 < total) relax_round<WT, 1>(a, t, u, du, s, excl, total, k0, nc, imp, loc);
 }
-
 
 }  // namespace gbs

@@ -19,8 +19,8 @@
 namespace gbs {
 
 // Who executes a phase: the CTA group (the whole grid for a single-source
-// launch) or one CTA.  Lists are dealt to warps in chunks of 32 entries (one
-// per lane), and the warps of a group are numbered CTA-minor: chunk c goes to
+// launch) or one CTA.  Lists are dealt to warps in chunks of entries (one per
+// lane), and the warps of a group are numbered CTA-minor: chunk c goes to
 // CTA c % group_ctas, so a phase of a few thousand entries runs one warp on
 // each of many SMs instead of 32 warps on each of a few (one SM issues every
 // load and atomic of its warps; on the 4096^2 grid, whose buckets start with
@@ -28,7 +28,26 @@ namespace gbs {
 struct Exec {
     uint32_t tid, nthreads;   // thread index and count over the executors (vertex loops)
     uint32_t warp, nwarps;    // warp index (CTA-minor in a group) and count over the executors
+    uint32_t least;           // fewest entries of a scan worth a warp of its own
 };
+
+// Entries a warp takes at a time in a scan of `count`: its share, at most one
+// per lane.  Most scans are smaller than 32 entries a warp, and what bounds
+// them is the chain of dependent loads and atomics of the busiest warp: with
+// fixed chunks of 32 a scan of 100 entries kept 4 of a CTA's 28 warps busy
+// (their rows take several rounds of 128 edges each), one of 8,000 entries 250
+// of the grid's 4,256.  The rows of a chunk are spread over all 32 lanes
+// whatever its size, so smaller chunks mean fewer rounds, not idle lanes.  The
+// grid stops at kLeastDeal entries because every warp pays global atomics on
+// the list counters; one CTA's counters are in its shared memory.  Kernel us,
+// chunks of 32 / grid at least 4, 8, 16 (one CTA: 1): R-MAT of 65,536
+// vertices 624 / 557, 563, 578, of 200,003 826 / 770, 776, 788, of 4.2 M
+// 1886 / 1822, 1812, 1846, 4096^2 grid 139,518 / 104,638, 105,679, 111,755.
+constexpr uint32_t kLeastDeal = 8u;
+__device__ __forceinline__ uint32_t deal_size(const Exec &x, uint32_t count) {
+    const uint32_t share = (count + x.nwarps - 1u) / x.nwarps;
+    return share < x.least ? x.least : (share > 32u ? 32u : share);
+}
 
 __device__ __forceinline__ uint32_t group_rank(const SsspArgs &a) {
     return blockIdx.x - a.group * a.group_ctas;
@@ -40,6 +59,7 @@ __device__ __forceinline__ Exec group_exec(const SsspArgs &a) {
     x.nthreads = a.group_ctas * blockDim.x;
     x.warp = (threadIdx.x >> 5) * a.group_ctas + group_rank(a);
     x.nwarps = x.nthreads >> 5;
+    x.least = kLeastDeal;
     return x;
 }
 
@@ -49,6 +69,7 @@ __device__ __forceinline__ Exec cta_exec() {
     x.nthreads = blockDim.x;
     x.warp = x.tid >> 5;
     x.nwarps = x.nthreads >> 5;
+    x.least = 1u;
     return x;
 }
 
@@ -164,7 +185,7 @@ __device__ __forceinline__ void fuse_drain(const SsspArgs &a, const Targets &t, 
     }
 }
 
-// One thread per frontier entry.  vtag != kTagInit keeps only entries whose
+// One lane per frontier entry.  vtag != kTagInit keeps only entries whose
 // tag equals it (ring lists may hold entries that moved to a lower bucket).
 // The scan relaxes the light prefix [row, mid) of each row, or the whole row
 // when full.  With a split, a vertex scanned for the first time in the
@@ -179,12 +200,13 @@ __device__ void scan_frontier(const SsspArgs &a, const Targets &t, const Exec &x
     uint32_t my_edges = 0;
     uint32_t nc = 0;   // candidates buffered by this warp
     Local loc{kNoLocal, 0u};
-    for (uint32_t base = x.warp * 32u; base < count; base += x.nthreads) {
+    const uint32_t deal = deal_size(x, count);
+    for (uint32_t base = x.warp * deal; base < count; base += x.nwarps * deal) {
         const uint32_t i = base + lane;
         uint32_t u = 0, s = 0, e = 0, he = 0;
         typename Arith<WT>::D du = 0;
         bool ok = false;
-        if (i < count) {
+        if (lane < deal && i < count) {
             u = __ldcg(F + i);
             // the tag check and the row reads are independent: issue together
             const uint32_t tg = (vtag == kTagInit) ? vtag : __ldcg(a.ws.tag + u);
