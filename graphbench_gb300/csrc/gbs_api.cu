@@ -538,6 +538,7 @@ gbs_status launch_run(gbs_graph *g, uint32_t src, const gbs_params *p, void *dis
     a.inline_max = (p && p->inline_edges) ? p->inline_edges : kInlineEdges;
     a.full_items = (p && p->full_items) ? p->full_items : std::max(g->n, kFullItems);
     a.fuse_rounds = (a.flags & GBS_F_NO_FUSE) ? 0u : ((p && p->fuse_rounds) ? p->fuse_rounds : kFuseRounds);
+    merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, learned, a.merge_low, a.merge_drain);
     a.run_ns = a.wait_ns * 16ull;
     a.ctrl = learned ? kCtrlLearned : kCtrlFixed;
     a.span_fixed = 1;
@@ -789,6 +790,8 @@ gbs_status gbs_graph_create(uint32_t n, uint64_t m, const uint64_t *row_offsets,
         wsum += wtype == GBS_WEIGHT_U32   ? (double)((const uint32_t *)weights)[e]
                 : wtype == GBS_WEIGHT_F32 ? (double)((const float *)weights)[e]
                                           : ((const double *)weights)[e];
+    uint32_t max_deg = 0;
+    for (uint32_t v = 0; v < n; ++v) max_deg = std::max(max_deg, row32[v + 1] - row32[v]);
     bool zero_w = false;
     // rows are sorted by weight: a zero weight is the first of its row
     for (uint32_t v = 0; v < n && !zero_w; ++v)
@@ -797,6 +800,7 @@ gbs_status gbs_graph_create(uint32_t n, uint64_t m, const uint64_t *row_offsets,
     gbs_graph *g = nullptr;
     st = graph_shell(n, m, wtype, max_w, m ? wsum / (double)m : 0.0, zero_w, &g);
     if (st != GBS_OK) return st;
+    g->max_deg = max_deg;
     cudaError_t e;
     if ((e = cudaMalloc(&g->d_row, sizeof(uint32_t) * (n + 1))) != cudaSuccess ||
         (e = cudaMalloc(&g->d_adj, sizeof(uint2) * (m ? m : 1))) != cudaSuccess ||

@@ -27,6 +27,7 @@ struct gbs_pack {
     std::vector<uint32_t> n;
     std::vector<uint64_t> m;
     std::vector<double> max_w;
+    std::vector<uint32_t> max_deg;
     std::vector<uint64_t> voff;   // count+1: first vertex of each graph in pack-wide arrays
     std::vector<uint64_t> eoff;   // count+1: first edge of each graph
     uint32_t *d_row = nullptr;    // graph i's n_i + 1 offsets start at voff[i] + i
@@ -281,6 +282,7 @@ gbs_status gbs_pack_create(uint32_t count, const gbs_csr_view *graphs, gbs_weigh
     p->n.resize(count);
     p->m.resize(count);
     p->max_w.resize(count);
+    p->max_deg.assign(count, 0);
     p->voff.assign(count + 1, 0);
     p->eoff.assign(count + 1, 0);
     for (uint32_t i = 0; i < count; ++i) {
@@ -308,6 +310,7 @@ gbs_status gbs_pack_create(uint32_t count, const gbs_csr_view *graphs, gbs_weigh
         }
         p->n[i] = v.n;
         p->m[i] = v.m;
+        for (uint32_t r = 0; r < v.n; ++r) p->max_deg[i] = std::max(p->max_deg[i], row32[r + 1] - row32[r]);
         if ((e = cudaMemcpy(p->d_row + p->voff[i] + i, row32.data(), sizeof(uint32_t) * (v.n + 1),
                             cudaMemcpyHostToDevice)) != cudaSuccess ||
             (v.m && (e = cudaMemcpy(p->d_adj + p->eoff[i], adj.data(), sizeof(uint2) * v.m,
@@ -377,6 +380,7 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
         d.delta_u = r.delta_u;
         d.inv_delta_f = r.inv_delta_f;
         d.no_heavy = no_heavy ? 1u : 0u;
+        merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, false, d.merge_low, d.merge_drain);
         d.dist = dist_dev ? static_cast<uint32_t *>(dist_dev) + (size_t)i * g->n : nullptr;
         d.pred = pred_dev ? pred_dev + (size_t)i * g->n : nullptr;
     }
@@ -441,6 +445,7 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
         d.delta_u = rs[i].delta_u;
         d.inv_delta_f = rs[i].inv_delta_f;
         d.no_heavy = nh[i] ? 1u : 0u;
+        merge_limits(pk->wtype, pk->n[i], pk->m[i], pk->max_deg[i], pk->max_w[i], false, d.merge_low, d.merge_drain);
         d.dist = dist_dev ? static_cast<uint32_t *>(dist_dev) + pk->voff[i] : nullptr;
         d.pred = pred_dev ? pred_dev + pk->voff[i] : nullptr;
         n_cap = std::max(n_cap, pk->n[i]);

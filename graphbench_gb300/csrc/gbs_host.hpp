@@ -34,6 +34,7 @@ struct gbs_graph {
     gbs_weight_type wtype = GBS_WEIGHT_U32;
     double max_w = 0.0;
     bool zero_w = false;                    // some edge weighs 0
+    uint32_t max_deg = 0;                   // edges of the longest row
     int device = 0;
     int sms = 0;
     cudaStream_t stream = nullptr;

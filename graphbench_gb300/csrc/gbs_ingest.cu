@@ -287,9 +287,16 @@ __global__ void k_adj(const uint32_t *__restrict__ id, const uint32_t *__restric
     }
 }
 
-__global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, uint32_t *__restrict__ row32) {
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
+// max_deg: raised to the longest row
+__global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, uint32_t *__restrict__ row32,
+                        uint32_t *max_deg) {
+    uint32_t d = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
         row32[v] = (uint32_t)row[v];
+        if (v < n) d = max(d, (uint32_t)(row[v + 1] - row[v]));
+    }
+    d = __reduce_max_sync(0xffffffffu, d);
+    if ((threadIdx.x & 31u) == 0) atomicMax(max_deg, d);
 }
 
 // ----------------------------------------------------------------- host
@@ -698,9 +705,9 @@ gbs_status graph_from_csr(const gbs_device_csr *c, gbs_weight_type wtype, gbs_gr
     uint32_t *row_of = nullptr, *flags = nullptr, *id0 = nullptr, *id1 = nullptr, *col_s = nullptr;
     unsigned long long *wbits = nullptr, *key = nullptr, *key_s = nullptr;
     ING_CUDA(bufs.get(&row_of, m));
-    ING_CUDA(bufs.get(&flags, 1));
+    ING_CUDA(bufs.get(&flags, 2));   // weight flags, longest row
     ING_CUDA(bufs.get(&wbits, m));
-    ING_CUDA(cudaMemsetAsync(flags, 0, sizeof(uint32_t), s));
+    ING_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), s));
     k_row_of<<<std::max(1, std::min<int>((n + 7) / 8, sms * 16)), 256, 0, s>>>(c->d_row, n, row_of);
     ING_CUDA(cudaGetLastError());
     if (wtype == GBS_WEIGHT_F64) k_weight_bits<2><<<gb, 256, 0, s>>>(c->d_w, m, wbits, flags);
@@ -770,9 +777,11 @@ gbs_status graph_from_csr(const gbs_device_csr *c, gbs_weight_type wtype, gbs_gr
         free_graph(g);
         return fail(e == cudaErrorMemoryAllocation ? GBS_ERR_NO_MEMORY : GBS_ERR_CUDA, cudaGetErrorString(e));
     }
-    k_row32<<<std::max(1, std::min<int>((n + 256) / 256, sms * 8)), 256, 0, s>>>(c->d_row, n, g->d_row);
+    k_row32<<<std::max(1, std::min<int>((n + 256) / 256, sms * 8)), 256, 0, s>>>(c->d_row, n, g->d_row, flags + 1);
     k_adj<<<gb, 256, 0, s>>>(id1, c->d_col, wbits, m, wtype == GBS_WEIGHT_F64, g->d_adj, g->d_w64);
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+    if ((e = cudaGetLastError()) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&g->max_deg, flags + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess) {
         free_graph(g);
         return fail(GBS_ERR_CUDA, cudaGetErrorString(e));
     }

@@ -133,6 +133,11 @@ struct __align__(128) Ctl {
     unsigned long long st_reached;
     unsigned long long st_edges_reached;
     unsigned long long inst_t0;   // globaltimer when the current instance started
+    // what the bucket merge knows of the run so far (kSLong .. kSWindow)
+    uint32_t st_long;
+    uint32_t st_entries;
+    uint32_t st_done;
+    uint32_t st_window;
 };
 static_assert(sizeof(Ctl) % 128 == 0, "Ctl lines");
 
@@ -140,8 +145,9 @@ static_assert(sizeof(Ctl) % 128 == 0, "Ctl lines");
 // index.  A phase run by the whole grid reaches them in global memory, one
 // Line apart; the deciding CTA keeps a copy in its shared memory while it
 // decides and while it runs phases alone, one word apart, and writes it back
-// before it releases the other CTAs.  Four statistics words follow the
-// counters in the shared copy (their global homes are the st_* fields).
+// before it releases the other CTAs.  Four statistics words and the four the
+// bucket merge reads follow the counters in the shared copy (their global
+// homes are the st_* fields).
 enum CtrIdx : uint32_t {
     kCRing = 0,
     kCFq = kNB,
@@ -155,6 +161,10 @@ enum CtrIdx : uint32_t {
     kSBuckets,
     kSPending,
     kSSolo,
+    kSLong,       // edges of long rows the current bucket's scans handed to EDGES
+    kSEntries,    // entries the last bucket started with
+    kSDone,       // entries all buckets so far started with
+    kSWindow,     // entries queued in the window and beyond it when the last bucket started
     kCtrShared,
 };
 static_assert(offsetof(Ctl, fq_cnt) == offsetof(Ctl, ring_cnt) + 128 * kCFq, "counter order");
@@ -203,6 +213,8 @@ struct InstDesc {
     uint32_t delta_u;
     float inv_delta_f;
     uint32_t no_heavy;
+    uint32_t merge_low;     // as SsspArgs.merge_low
+    uint32_t merge_drain;   // as SsspArgs.merge_drain
     uint32_t *dist;
     int32_t *pred;
 };
@@ -246,6 +258,9 @@ struct SsspArgs {
     uint32_t full_items;    // kCtrlFixed: a bucket whose lists hold at most this many entries when it
                             // starts relaxes whole rows (no heavy phase)
     uint32_t fuse_rounds;   // bucket fusion rounds per warp in whole-row scans (0: none)
+    uint32_t merge_low;     // a bucket takes in the next base buckets while their lists hold at most
+                            // this many entries (0: no such merge; see merge_spans)
+    uint32_t merge_drain;   // base buckets a bucket takes in while the run drains (0 or 1: none)
     // bucket-width controller
     uint32_t ctrl;          // CtrlMode
     uint32_t span_fixed;    // kCtrlFixed: base widths per bucket (0 or 1 = plain delta-stepping)

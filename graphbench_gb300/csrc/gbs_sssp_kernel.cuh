@@ -67,6 +67,49 @@ constexpr uint32_t kFullItems = 1024u;           // least split threshold
 // 4096^2 grid 209.6 -> 209.7.
 inline uint32_t split_full_items(uint32_t n) { return n / 16u > kFullItems ? n / 16u : kFullItems; }
 
+// Bucket merge (decide_bucket): a bucket starts with the lists of several
+// base buckets at once when they are too thin to fill the machine.  The run
+// then takes fewer dependent phases; the least fixpoint is the same for every
+// span.  Two rules, either of which may widen a bucket:
+//   low    graphs without long rows (road networks, grids, meshes), whose
+//          frontier grows by at most the degree a hop: the next base buckets
+//          while they hold at most kMergeEdges edges (entries x average degree)
+//          together, up to kMergeLow of them
+//   drain  the run has started 1/16 of the vertices, and either the last
+//          bucket relaxed fewer edges of long rows than it had entries or the
+//          queues shrank over it: what is left are short rows that improve
+//          little, so up to kMergeDrain base buckets go together, whatever
+//          they hold (kMergeLearned in a learned run)
+// Merging while a skewed graph still reaches its hubs relaxes their rows again
+// and again: R-MAT 22 with 8 thin base buckets merged from the start 1.83 ->
+// 2.85 ms.  Kernel ms, no merge -> these rules (longest row): uniform random
+// graph of 1 M vertices and degree 8 (25) 0.88 -> 0.71, 16 (39) 1.17 -> 0.99,
+// lattice with random short links, 1 M (20) 16.8 -> 9.6, 1024^2 grid (4) 28.5
+// -> 10.5, R-MAT 16 (6,299) 0.47 -> 0.35, 18 0.74 -> 0.47, 20 1.05 -> 0.73,
+// 22 (162,304) 1.97 -> 1.60.  A drain of 8 or 16 base buckets gains a little
+// more (R-MAT 20 0.64, 0.61; 22 1.48, 1.43); a learned run, whose base widths
+// the controller picks, takes up to 32.
+constexpr uint32_t kMergeEdges = 131072u;
+constexpr uint32_t kMergeLow = 16u;
+constexpr uint32_t kMergeDrain = 4u;
+constexpr uint32_t kMergeLearned = 32u;
+constexpr uint32_t kMergeMax = 32u;          // one lane per list of a merged bucket
+
+// The two limits of a graph.  uint32 sums: a vertex of a merged bucket relaxes
+// its row from a distance that may lie up to the bucket's width above its
+// final one, so a sum could pass 2^32 - 1 that does not in the end; where no
+// path can (n x the largest weight below it) buckets merge, elsewhere not.
+inline void merge_limits(gbs_weight_type wt, uint32_t n, uint64_t m, uint32_t max_deg, double max_w, bool learned,
+                         uint32_t &low, uint32_t &drain) {
+    low = drain = 0u;
+    if (n == 0 || (wt == GBS_WEIGHT_U32 && (double)n * max_w >= 4294967295.0)) return;
+    if (max_deg <= kInlineEdges) {
+        const uint64_t avg = (m + n - 1) / n;
+        low = kMergeEdges / (uint32_t)(avg ? avg : 1);
+    }
+    drain = learned ? kMergeLearned : kMergeDrain;
+}
+
 // Values identical in every CTA (the kernel's uniform state).
 struct Uniform {
     uint32_t phase;       // phase being executed

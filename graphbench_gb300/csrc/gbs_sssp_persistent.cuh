@@ -82,6 +82,10 @@ __device__ __forceinline__ uint32_t *counter_home(Ctl *ctl, uint32_t i) {
         case kSBuckets: return &ctl->st_buckets;
         case kSPending: return &ctl->st_pending_scans;
         case kSSolo: return &ctl->st_solo_phases;
+        case kSLong: return &ctl->st_long;
+        case kSEntries: return &ctl->st_entries;
+        case kSDone: return &ctl->st_done;
+        case kSWindow: return &ctl->st_window;
         default: return global_ctrs(ctl).at(i);
     }
 }
@@ -191,9 +195,14 @@ __device__ __forceinline__ void fuse_drain(const SsspArgs &a, const Targets &t, 
 // when full.  With a split, a vertex scanned for the first time in the
 // current heavy round also emits descriptors for its heavy edges [mid, end):
 // the HEAVY phase relaxes them once the bucket's light loop has settled.
+// A bucket of several base buckets (span > 1) hands over their lists as one:
+// F is null, vtag the first base bucket and excl lane j's exclusive prefix of
+// the lists' sizes, so short lists share the warps instead of running one
+// after the other.
 template <int WT>
 __device__ void scan_frontier(const SsspArgs &a, const Targets &t, const Exec &x, const uint32_t *F,
-                              uint32_t count, uint32_t vtag, bool full, uint32_t hround, uint32_t &imp) {
+                              uint32_t count, uint32_t vtag, bool full, uint32_t hround, uint32_t &imp,
+                              uint32_t span = 1u, uint32_t excl = 0u) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = lane_id();
     Ctl *ctl = a.ws.ctl;
@@ -206,15 +215,27 @@ __device__ void scan_frontier(const SsspArgs &a, const Targets &t, const Exec &x
         uint32_t u = 0, s = 0, e = 0, he = 0;
         typename Arith<WT>::D du = 0;
         bool ok = false;
+        uint32_t want = vtag;
+        const uint32_t *at = F + i;
+        if (span > 1u) {
+            uint32_t own = 0;   // the last list whose prefix is at most i
+#pragma unroll
+            for (uint32_t b = 16; b > 0; b >>= 1) {
+                const uint32_t ex = __shfl_sync(FULL, excl, own + b);
+                if (own + b < span && ex <= i) own += b;
+            }
+            want = vtag + own;
+            at = a.ws.ring + (size_t)(want % kNB) * a.g.n + (i - __shfl_sync(FULL, excl, own));
+        }
         if (lane < deal && i < count) {
-            u = __ldcg(F + i);
+            u = __ldcg(at);
             // the tag check and the row reads are independent: issue together
             const uint32_t tg = (vtag == kTagInit) ? vtag : __ldcg(a.ws.tag + u);
             du = dist_of<WT>(__ldcg(a.ws.dp + u));
             const uint32_t r = __ldg(a.g.row + u);
             const uint32_t re = __ldg(a.g.row + u + 1);
             const uint32_t md = full ? re : __ldg(a.ws.mid + u);
-            ok = tg == vtag;
+            ok = tg == want;
             s = ok ? r : 0u;
             e = ok ? md : 0u;
             he = ok ? re : 0u;
@@ -466,13 +487,20 @@ __device__ void run_phase(const SsspArgs &a, const Uniform &U, const Exec &x, Wa
     const bool pub = U.items != kNoItems;
     switch (U.phase) {
         case kPhLightFirst:
-            // the ring lists of every base bucket the bucket spans, one after
-            // the other (independent: no barrier between them)
-            for (uint32_t j = 0; j < U.span; ++j) {
-                const uint32_t bk = U.b + j;
-                const uint32_t cnt = (pub && U.span == 1u) ? U.items : ld_relaxed_any(c.at(kCRing + bk % kNB));
-                scan_frontier<WT>(a, t, x, a.ws.ring + (size_t)(bk % kNB) * n, min(cnt, n), bk, full, U.hround,
-                                  imp);
+            if (U.span == 1u) {
+                const uint32_t cnt = pub ? U.items : ld_relaxed_any(c.at(kCRing + U.b % kNB));
+                scan_frontier<WT>(a, t, x, a.ws.ring + (size_t)(U.b % kNB) * n, min(cnt, n), U.b, full, U.hround, imp);
+            } else {   // the ring lists of every base bucket the bucket spans (at most kMergeMax)
+                const unsigned lane = lane_id();
+                const uint32_t len = lane < U.span ? min(ld_relaxed_any(c.at(kCRing + (U.b + lane) % kNB)), n) : 0u;
+                uint32_t incl = len;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if ((int)lane >= o) incl += y;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                scan_frontier<WT>(a, t, x, nullptr, total, U.b, full, U.hround, imp, U.span, incl - len);
             }
             break;
         case kPhLight:
@@ -554,10 +582,13 @@ __device__ __forceinline__ void mlp_eval(const float *__restrict__ P, const floa
 // of the lists it spans (warp-collective: warp 0 of the deciding CTA).  The
 // fixed schedule keeps span_fixed base widths; the learned one evaluates the
 // controller on the occupancy of the next base buckets, the run so far and
-// the graph.  GBS_F_FEATURES records the controller input.
+// the graph.  Either may be widened by the bucket merge (gbs_sssp_kernel.cuh);
+// GBS_F_FEATURES records the controller input, for the widths the caller asked
+// for: such a run does not merge.
 __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const uint32_t *sc, uint32_t nb, uint32_t lim,
                                               uint32_t ring_lo, uint32_t ring_hi, uint32_t pend, uint32_t pm,
-                                              uint32_t &span_out, uint32_t &full_out, uint32_t &first_items) {
+                                              uint32_t entries, uint32_t done, uint32_t &span_out, uint32_t &full_out,
+                                              uint32_t &first_items, uint32_t &window) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = lane_id();
     auto ring_count = [&](uint32_t bucket) {
@@ -622,6 +653,24 @@ __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const
             span = 1u << e;
             full = (a.no_heavy || y1 <= 0.f) ? 1u : 0u;   // y1: logit of "split at the light bound"
         }
+    }
+    window = c_lo + c_hi;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) window += __shfl_xor_sync(FULL, window, o);
+    window += pend;
+    if (!want_feat) {
+        const bool quiet = sc[kSLong] <= entries, shrinks = window < sc[kSWindow];
+        uint32_t wide = (done >= a.g.n / 16u && (quiet || shrinks)) ? a.merge_drain : 0u;
+        if (a.merge_low) {
+            uint32_t incl = c_lo;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, incl, o);
+                if ((int)lane >= o) incl += y;
+            }
+            wide = max(wide, (uint32_t)__popc(__ballot_sync(FULL, lane < kMergeLow && incl <= a.merge_low)));
+        }
+        span = max(span, wide);
     }
     // a bucket never reaches past the smallest pending bucket
     while (span > 1u && pend > 0u && nb + span > pm) span >>= 1;
@@ -780,11 +829,14 @@ __device__ inline void control_step(const SsspArgs &a, const Uniform &U, bool wa
             N.hround = 1u;
         }
     }
+    uint32_t window = 0;        // LIGHT_FIRST: entries queued anywhere
     uint32_t first_items = 0;   // LIGHT_FIRST: entries of every list the new bucket spans
     if (next == kPhLightFirst) {
         uint32_t span, full;
-        decide_bucket(a, ctl, sc, nb, U.W + kNB, ring_lo, ring_hi, ps2 ? pc1 : pc0, ps2 ? pm1 : pm0, span, full,
-                      first_items);
+        const bool first = U.phase == kPhLightFirst;
+        decide_bucket(a, ctl, sc, nb, U.W + kNB, ring_lo, ring_hi, ps2 ? pc1 : pc0, ps2 ? pm1 : pm0,
+                      first ? cur_ring : sc[kSEntries], sc[kSDone] + (first ? cur_ring : 0u), span, full, first_items,
+                      window);
         N.span = span;
         N.full = full;
     }
@@ -852,7 +904,16 @@ __device__ inline void control_step(const SsspArgs &a, const Uniform &U, bool wa
             a.res[U.inst] = r;
         }
         if (U.phase < kPhDone) sc[kSPhases] += 1;
-        if (U.phase == kPhLightFirst) sc[kSBuckets] += 1;
+        if (U.phase == kPhLightFirst) {
+            sc[kSBuckets] += 1;
+            sc[kSEntries] = cur_ring;
+            sc[kSDone] += cur_ring;
+        }
+        if (U.phase == kPhLightFirst || U.phase == kPhLight) sc[kSLong] += edge_cnt;
+        if (next == kPhLightFirst) {
+            sc[kSLong] = 0;
+            sc[kSWindow] = window;
+        }
         if (U.phase == kPhPending) {
             sc[kSPending] += 1;
             sc[kCPend + U.pend_sel] = 0;          // the list just re-bucketed
@@ -902,6 +963,10 @@ __device__ inline void control_step(const SsspArgs &a, const Uniform &U, bool wa
             sc[kSPhases] = 0u;
             sc[kSPending] = 0u;
             sc[kSSolo] = 0u;
+            sc[kSLong] = 0u;
+            sc[kSEntries] = 0u;
+            sc[kSDone] = 0u;
+            sc[kSWindow] = 0u;
             ctl->st_improvements = 0ull;
             ctl->st_reached = 0ull;
             ctl->st_edges_reached = 0ull;
@@ -1136,6 +1201,8 @@ __global__ void __launch_bounds__(kTPB, 1) sssp_batch(SsspArgs base, const Works
                 s_a.delta_u = d.delta_u;
                 s_a.inv_delta_f = d.inv_delta_f;
                 s_a.no_heavy = d.no_heavy;
+                s_a.merge_low = d.merge_low;
+                s_a.merge_drain = d.merge_drain;
                 s_a.dist_out = d.dist;
                 s_a.pred_out = d.pred;
             }

@@ -64,7 +64,8 @@ typedef struct gbs_graph gbs_graph;
 typedef struct gbs_params {
     double delta;            /* bucket width; <= 0 selects max_w / average out-degree
                                 (the published configs' rule).  uint32 graphs use
-                                floor(delta), at least 1. */
+                                floor(delta), at least 1.  Buckets too thin to fill
+                                the GPU are processed several at a time. */
     double light;            /* light/heavy split: an edge is light iff w <= light.
                                 < 0 selects light = delta (the reference's rule,
                                 graph/csr.c:84). */
