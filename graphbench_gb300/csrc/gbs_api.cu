@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "gbs_host.hpp"
+#include "gbs_small.cuh"
 
 using namespace gbs;
 
@@ -349,6 +350,8 @@ void free_graph(gbs_graph *g) {
     cudaFree(g->d_pred);
     cudaFree(g->d_mlp);
     cudaFree(g->d_feat);
+    cudaFreeHost(g->h_small);
+    cudaFreeHost(g->h_stage);
     free_bc(g);
     for (auto &e : g->ev) if (e) cudaEventDestroy(e);
     if (g->stream) cudaStreamDestroy(g->stream);
@@ -665,6 +668,9 @@ gbs_status launch_run(gbs_graph *g, uint32_t src, const gbs_params *p, void *dis
 // call made.
 gbs_status run_sssp(gbs_graph *g, uint32_t src, const gbs_params *p, void *dist_dev, int32_t *pred_dev,
                     gbs_stats *stats) {
+    // without an output the caller wants the state words of the workspace
+    if ((dist_dev || pred_dev) && small_call(g, p))
+        return small_run(g, src, dist_dev, pred_dev, !(p && (p->flags & GBS_F_NO_STATS)), stats);
     const bool learned = p && (p->flags & GBS_F_LEARNED);
     if (!learned) return launch_run(g, src, p, dist_dev, pred_dev, stats, false, nullptr);
     if (!g->d_mlp) return fail(GBS_ERR_INVALID_ARG, "GBS_F_LEARNED: no controller set (gbs_graph_set_controller)");
@@ -865,7 +871,20 @@ gbs_status gbs_sssp(gbs_graph *g, uint32_t source, const gbs_params *params, voi
     void *pred_view = device_view(pred_out);
     if ((!dist_out || dist_view) && (!pred_out || pred_view) && (dist_out || pred_out))
         return run_sssp(g, source, params, dist_view, static_cast<int32_t *>(pred_view), stats);
-    gbs_status st = ensure_workspace(g);
+    gbs_status st;
+    if ((dist_out || pred_out) && small_call(g, params)) {
+        // a small graph's results reach pageable memory through a page-locked
+        // buffer the kernel writes: no device buffers, no copies to wait for
+        const size_t b = sizeof(uint32_t) * (size_t)g->n;
+        if (!g->h_stage) GBS_CUDA(cudaMallocHost(&g->h_stage, 2 * b));
+        st = run_sssp(g, source, params, dist_out ? g->h_stage : nullptr,
+                      pred_out ? reinterpret_cast<int32_t *>(g->h_stage + b) : nullptr, stats);
+        if (st != GBS_OK) return st;
+        if (dist_out) std::memcpy(dist_out, g->h_stage, b);
+        if (pred_out) std::memcpy(pred_out, g->h_stage + b, b);
+        return GBS_OK;
+    }
+    st = ensure_workspace(g);
     if (st != GBS_OK) return st;
     st = run_sssp(g, source, params, dist_out ? g->d_dist : nullptr, pred_out ? g->d_pred : nullptr,
                     stats);

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "gbs_host.hpp"
+#include "gbs_small.cuh"
 
 using namespace gbs;
 
@@ -92,6 +93,38 @@ void free_pack(gbs_pack *p) {
     cudaFree(p->d_row);
     cudaFree(p->d_adj);
     delete p;
+}
+
+// Whether every knob of a plan is at its default.
+bool default_plan(const gbs_batch_params *bp) {
+    return !bp || (!(bp->delta > 0) && !(bp->delta_scale > 0) && !(bp->light >= 0) && !bp->group_ctas && !bp->flags &&
+                   !bp->solo_entries && !bp->solo_descs && !bp->inline_edges && !bp->fuse_rounds);
+}
+
+// A plan whose instances are all solved by one CTA each (gbs_small.cu): no
+// workspaces, and the launch needs no co-resident groups.
+gbs_status build_small_plan(gbs_plan *p, int sms, uint32_t n_cap, uint64_t m_cap, const std::vector<InstDesc> &inst) {
+    p->count = (uint32_t)inst.size();
+    const SmallShape shape = small_shape(n_cap, m_cap);
+    p->groups = p->blocks = small_grid(p->f32, shape, sms, p->count);
+    p->group_ctas = 1;
+    if (!p->blocks) return fail(GBS_ERR_UNSUPPORTED, "one-CTA kernel cannot be resident");
+    GBS_CUDA(cudaMalloc(&p->d_inst, sizeof(InstDesc) * p->count));
+    GBS_CUDA(cudaMemcpyAsync(p->d_inst, inst.data(), sizeof(InstDesc) * p->count, cudaMemcpyHostToDevice, p->stream));
+    GBS_CUDA(cudaMalloc(&p->d_res, sizeof(InstResult) * p->count));
+    GBS_CUDA(cudaMemsetAsync(p->d_res, 0, sizeof(InstResult) * p->count, p->stream));
+    GBS_CUDA(cudaMalloc(&p->d_queue, sizeof(uint32_t)));
+    GBS_CUDA(cudaStreamSynchronize(p->stream));
+    p->host_res.resize(p->count);
+    GBS_CUDA(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
+    k_batch_prep<<<1, 256, 0, p->stream>>>(nullptr, 0, p->d_res, p->count, p->d_queue);
+    const gbs_status st = small_launch(p->f32, shape, p->blocks, p->d_inst, p->d_res, p->count, p->d_queue, p->stream);
+    const cudaError_t e = cudaStreamEndCapture(p->stream, &p->graph);
+    if (st != GBS_OK) return st;
+    GBS_CUDA(e);
+    GBS_CUDA(cudaGraphInstantiate(&p->exec, p->graph, 0));
+    GBS_CUDA(cudaGraphUpload(p->exec, p->stream));
+    return GBS_OK;
 }
 
 size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -354,7 +387,8 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
     const Resolved r = schedule_of(params, g->wtype, g->max_w, g->n, g->m);
     const bool no_heavy = r.light_bits >= max_weight_bits(g->wtype, g->max_w);
     const uint32_t *mid = g->d_row + 1;   // no split: the first heavy edge is the row end
-    if (!no_heavy) {
+    const bool small = default_plan(params) && small_graph(g->wtype, g->n, g->m, g->max_w, true);
+    if (!no_heavy && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * g->n);
         if (e != cudaSuccess) {
             free_plan(p);
@@ -384,7 +418,7 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
         d.dist = dist_dev ? static_cast<uint32_t *>(dist_dev) + (size_t)i * g->n : nullptr;
         d.pred = pred_dev ? pred_dev + (size_t)i * g->n : nullptr;
     }
-    st = build_plan(p, params, g->sms, g->n, g->m, inst);
+    st = small ? build_small_plan(p, g->sms, g->n, g->m, inst) : build_plan(p, params, g->sms, g->n, g->m, inst);
     if (st != GBS_OK) {
         free_plan(p);
         return st;
@@ -404,15 +438,16 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
     gbs_status st = new_plan(pk->device, pk->wtype == GBS_WEIGHT_F32, &p);
     if (st != GBS_OK) return st;
     std::vector<InstDesc> inst(pk->count);
-    bool any_split = false;
+    bool any_split = false, small = default_plan(params);
     std::vector<Resolved> rs(pk->count);
     std::vector<bool> nh(pk->count);
     for (uint32_t i = 0; i < pk->count; ++i) {
         rs[i] = schedule_of(params, pk->wtype, pk->max_w[i], pk->n[i], pk->m[i]);
         nh[i] = rs[i].light_bits >= max_weight_bits(pk->wtype, pk->max_w[i]);
         any_split = any_split || !nh[i];
+        small = small && small_graph(pk->wtype, pk->n[i], pk->m[i], pk->max_w[i], true);
     }
-    if (any_split) {
+    if (any_split && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * std::max<uint64_t>(pk->voff[pk->count], 1));
         if (e != cudaSuccess) {
             free_plan(p);
@@ -430,7 +465,7 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
         d.g.wtype = pk->wtype;
         d.g.row = row;
         d.g.adj = adj;
-        if (nh[i]) {
+        if (nh[i] || small) {
             d.mid = row + 1;
         } else {
             uint32_t *mid = p->d_mid + pk->voff[i];
@@ -457,7 +492,8 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
     std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return pk->m[x] > pk->m[y]; });
     std::vector<InstDesc> sorted(pk->count);
     for (uint32_t i = 0; i < pk->count; ++i) sorted[i] = inst[order[i]];
-    st = build_plan(p, params, pk->sms, n_cap, m_cap, sorted);
+    st = small ? build_small_plan(p, pk->sms, n_cap, m_cap, sorted)
+               : build_plan(p, params, pk->sms, n_cap, m_cap, sorted);
     if (st != GBS_OK) {
         free_plan(p);
         return st;

@@ -63,6 +63,10 @@ struct gbs_graph {
     // recorded controller inputs (GBS_F_FEATURES)
     float *d_feat = nullptr;
     uint32_t feat_cap = 0, feat_n = 0;
+    // graphs solved by one CTA (gbs_small.cu), page-locked, allocated on first
+    // use: the statistics of a run, and dist | pred for pageable outputs
+    gbs::InstResult *h_small = nullptr;
+    unsigned char *h_stage = nullptr;
     // betweenness state (gbs_bc), allocated on first use
     void *bc = nullptr;
 };

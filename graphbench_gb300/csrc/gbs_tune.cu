@@ -37,19 +37,22 @@ struct Budget {
     bool left() const { return used_ms < limit_ms; }
 };
 
-// Mean kernel time per source of one schedule (one untimed warm-up run).
+// Mean kernel time per source of one schedule (one untimed warm-up run), by
+// the path a call with these parameters and outputs takes.
 gbs_status time_single(gbs_graph *g, const std::vector<uint32_t> &src, const gbs_params &p, Budget &b,
                        uint32_t &runs, double &mean_ms) {
     gbs_stats st;
     gbs_params q = p;
     q.flags |= GBS_F_NO_STATS;
-    gbs_status s = gbs_sssp_device(g, src[0], &q, nullptr, nullptr, &st);
+    gbs_status s = ensure_workspace(g);
+    if (s != GBS_OK) return s;
+    s = gbs_sssp_device(g, src[0], &q, g->d_dist, g->d_pred, &st);
     if (s != GBS_OK) return s;
     ++runs;
     b.used_ms += st.kernel_ms;
     double sum = 0.0;
     for (uint32_t x : src) {
-        s = gbs_sssp_device(g, x, &q, nullptr, nullptr, &st);
+        s = gbs_sssp_device(g, x, &q, g->d_dist, g->d_pred, &st);
         if (s != GBS_OK) return s;
         ++runs;
         sum += st.kernel_ms;
