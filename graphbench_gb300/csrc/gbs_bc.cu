@@ -1,11 +1,12 @@
 // gbs_bc.cu -- betweenness centrality on the GPU (sm_103a): Brandes over the
 // shortest paths of every source, after btwcentral/csr_bc.c:16-123.
 //
-// Per source, the persistent delta-stepping kernel leaves the distances in
-// the graph's workspace; one cooperative launch of bc_dag then works on the
-// shortest-path DAG, the edges (u, v) with dist(u) + w == dist(v) computed in
-// the weight type (the reference keeps these as predecessor lists,
-// sssp/csr_sspath.c:116-118; here they are derived from the distances):
+// The shortest-path runs leave every source's distances on the device; a
+// cooperative launch of bc_dag then works on the shortest-path DAGs of several
+// sources at once, a group of CTAs and a set of arrays each.  A DAG is the edges
+// (u, v) with dist(u) + w == dist(v) computed in the weight type (the reference
+// keeps these as predecessor lists, sssp/csr_sspath.c:116-118; here they are
+// derived from the distances):
 //
 //   COUNT     every reached vertex: sigma := [v == source]; every tight
 //             out-edge (u, v) sets its bit in the tight-edge mask (one bit per
@@ -20,7 +21,16 @@
 //   BACKWARD  levels in reverse: every vertex pulls
 //             delta[u] = sum over tight out-edges (u, v) of
 //                        (1 + delta[v]) * sigma[u] / sigma[v]
-//             (comp_delta, csr_bc.c:93-116) and adds it to bc[u].
+//             (comp_delta, csr_bc.c:93-116).
+// After the launch k_bc_sum adds the sources' dependencies to bc, in the order
+// of the sources (a launch of one source adds its own).
+//
+// A source alone cannot fill the GPU on a graph of a few hundred thousand
+// vertices: its passes are some 40 levels of a grid barrier and a chain of L2
+// round trips each (R-MAT of 131,071 vertices: 0.41 ms a source on 152 CTAs).
+// Groups run as many sources at once as keep their arrays in L2 (bc_groups);
+// 16 sources: of that graph 6.0 -> 1.2 ms, of an R-MAT 20 16.1 -> 9.0, 8 of a
+// 300 x 400 grid 65 -> 8.7.
 //
 // Work layout.  A level is the slice order[lo, hi) of one order list.  Rows
 // of at most kLaneRow edges (two mask words) are walked by one lane.  A longer
@@ -97,7 +107,8 @@ struct BcArgs {
     const uint32_t *row;
     const uint2 *adj;
     const unsigned long long *w64;
-    const unsigned long long *dp;    // the SSSP's state words: distance (| pred)
+    const void *state;               // distances: uint32 / float32 values of a batched run, or the
+                                     // single-source kernel's state words (distance, | pred)
     uint32_t n;
     uint32_t source;
     unsigned long long *sigma;
@@ -120,13 +131,13 @@ struct BcArgs {
                                      //   first position, bit p set if a row starts at position p > 0}
     uint32_t n_words;                // mask words holding positions (m / 32 rounded up)
     uint32_t m;
-    double *bc;
+    double *bc;                      // one source at a time: takes its dependencies (else k_bc_sum adds them)
     BcCtl *ctl;
     BcTotals *tot;
     TraceRec *trace;                 // GBS_F_TRACE: one record per phase (kinds kTrCount..kTrBackward)
     uint32_t trace_cap;
     unsigned long long wait_ns;
-    uint32_t nblocks;
+    uint32_t nblocks;                // CTAs of the group
 };
 
 // Trace record kinds of the betweenness phases (bucket = level, items =
@@ -153,18 +164,34 @@ __device__ __forceinline__ void trace_phase(const BcArgs &a, uint32_t kind, uint
     c->trace_n = i + 1;
 }
 
-// dist(u) + w(e) == dist(v) in the weight type (both state words reached).
+// How a source's distances are stored: Word, the single-source kernel's 64-bit
+// state words (float64: the distance alone); else 32-bit distances.
+template <int WT, bool Word>
+struct State {
+    using T = unsigned long long;
+    static constexpr T kNone = kUnreached;
+    __device__ static __forceinline__ uint32_t dist(T x) { return (uint32_t)(x >> 32); }
+};
 template <int WT>
-__device__ __forceinline__ bool tight(unsigned long long pu, unsigned long long pv, uint2 ew,
+struct State<WT, false> {
+    using T = uint32_t;
+    static constexpr T kNone = WT == 1 ? 0x7F800000u : 0xFFFFFFFFu;
+    __device__ static __forceinline__ uint32_t dist(T x) { return x; }
+};
+
+// dist(u) + w(e) == dist(v) in the weight type (both reached).
+template <int WT, bool Word>
+__device__ __forceinline__ bool tight(typename State<WT, Word>::T pu, typename State<WT, Word>::T pv, uint2 ew,
                                       const unsigned long long *w64, uint32_t e) {
+    using S = State<WT, Word>;
     if constexpr (WT == 2) {
         const double s = __dadd_rn(__longlong_as_double((long long)pu), __longlong_as_double((long long)__ldg(w64 + e)));
         return (unsigned long long)__double_as_longlong(s) == pv;
     } else if constexpr (WT == 1) {
-        const float s = __fadd_rn(__uint_as_float((uint32_t)(pu >> 32)), __uint_as_float(ew.y));
-        return __float_as_uint(s) == (uint32_t)(pv >> 32);
+        const float s = __fadd_rn(__uint_as_float(S::dist(pu)), __uint_as_float(ew.y));
+        return __float_as_uint(s) == S::dist(pv);
     } else {
-        return (unsigned long long)(uint32_t)(pu >> 32) + ew.y == (pv >> 32);
+        return (unsigned long long)S::dist(pu) + ew.y == S::dist(pv);
     }
 }
 
@@ -324,21 +351,29 @@ __device__ __forceinline__ unsigned long long ld_state_keep(const unsigned long 
     asm volatile("ld.global.nc.L2::cache_hint.u64 %0, [%1], %2;" : "=l"(v) : "l"(ptr), "l"(pol));
     return v;
 }
+__device__ __forceinline__ uint32_t ld_state_keep(const uint32_t *ptr, unsigned long long pol) {
+    uint32_t v;
+    asm volatile("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(ptr), "l"(pol));
+    return v;
+}
 
 // COUNT over mask words: the warp takes kCountUnroll words per round, one
 // position per lane, all loads of the round in flight before any is used.
 // The row owning position W * 32 + l is ne_rows[k0 + popc(starts & bits 1..l)].
 constexpr uint32_t kCountUnroll = 4;
-template <int WT>
+template <int WT, bool Word>
 __device__ __forceinline__ void count_words(const BcArgs &a, uint32_t W0, uint32_t stride,
                                             unsigned long long &tight_n) {
+    using S = State<WT, Word>;
+    using T = typename S::T;
+    const T *state = static_cast<const T *>(a.state);
     const unsigned lane = threadIdx.x & 31u;
     const uint32_t below = (2u << lane) - 1u;
     const unsigned long long pol_first = l2_policy_first(), pol_last = l2_policy_last();
     for (uint32_t Wb = W0; Wb < a.n_words; Wb += stride * kCountUnroll) {
         uint32_t e[kCountUnroll], u[kCountUnroll];
         uint2 ew[kCountUnroll];
-        unsigned long long pu[kCountUnroll], pv[kCountUnroll];
+        T pu[kCountUnroll], pv[kCountUnroll];
         bool ok[kCountUnroll];
 #pragma unroll
         for (uint32_t j = 0; j < kCountUnroll; ++j) {
@@ -357,12 +392,12 @@ __device__ __forceinline__ void count_words(const BcArgs &a, uint32_t W0, uint32
         for (uint32_t j = 0; j < kCountUnroll; ++j) u[j] = ok[j] ? __ldg(a.ne_rows + u[j]) : 0u;
 #pragma unroll
         for (uint32_t j = 0; j < kCountUnroll; ++j) {
-            pu[j] = ok[j] ? ld_state_keep(a.dp + u[j], pol_last) : kUnreached;
-            pv[j] = ok[j] ? ld_state_keep(a.dp + ew[j].x, pol_last) : kUnreached;
+            pu[j] = ok[j] ? ld_state_keep(state + u[j], pol_last) : S::kNone;
+            pv[j] = ok[j] ? ld_state_keep(state + ew[j].x, pol_last) : S::kNone;
         }
 #pragma unroll
         for (uint32_t j = 0; j < kCountUnroll; ++j)
-            if (pu[j] != kUnreached && pv[j] != kUnreached && tight<WT>(pu[j], pv[j], ew[j], a.w64, e[j])) {
+            if (pu[j] != S::kNone && pv[j] != S::kNone && tight<WT, Word>(pu[j], pv[j], ew[j], a.w64, e[j])) {
                 atomicAdd(a.indeg + ew[j].x, 1u);
                 atomicOr(a.mask + (e[j] >> 5), 1u << (e[j] & 31u));
                 ++tight_n;
@@ -486,6 +521,12 @@ __device__ __forceinline__ uint32_t flat_owner(uint32_t incl, uint32_t k) {
 __device__ __forceinline__ uint32_t nth_low_bit(unsigned long long x, uint32_t n) {
     for (uint32_t r = 0; r < n; ++r) x &= x - 1ull;
     return (uint32_t)(__ffsll((long long)x) - 1);
+}
+
+// The dependency of a finished vertex.
+__device__ __forceinline__ void put_delta(const BcArgs &a, uint32_t u, double d) {
+    a.delta[u] = d;
+    if (a.bc) a.bc[u] = __dadd_rn(a.bc[u], d);
 }
 
 // One dependency term (1 + delta[v]) * sigma[u] / sigma[v], in the order of
@@ -649,9 +690,7 @@ __device__ __forceinline__ void backward_rows(const BcArgs &a, uint32_t i0, uint
     const double p0 = word_sums(a, w0, b0, su);
     const double p1 = word_sums(a, w0 + 1, b1, su);
     if (mine) {
-        const double d = __dadd_rn(p0, p1);
-        a.delta[u] = d;
-        a.bc[u] = __dadd_rn(a.bc[u], d);
+        put_delta(a, u, __dadd_rn(p0, p1));
     }
 }
 
@@ -685,10 +724,7 @@ __device__ __forceinline__ void finish_row(const BcArgs &a, uint32_t bu, uint32_
         r = __dadd_rn(r, __shfl_sync(kFull, butterfly32(cur), 0));
         cur = next;
     }
-    if (lane == 0) {
-        a.delta[bu] = r;
-        a.bc[bu] = __dadd_rn(a.bc[bu], r);
-    }
+    if (lane == 0) put_delta(a, bu, r);
 }
 
 __device__ __forceinline__ void finish_rows(const BcArgs &a, uint32_t s0, uint32_t shi) {
@@ -708,8 +744,7 @@ __device__ __forceinline__ void finish_rows(const BcArgs &a, uint32_t s0, uint32
         for (uint32_t h = 4; h > 0; h >>= 1)
 #pragma unroll
             for (uint32_t k = 0; k < h; ++k) q[k] = __dadd_rn(q[k], q[k + h]);
-        a.delta[u] = q[0];
-        a.bc[u] = __dadd_rn(a.bc[u], q[0]);
+        put_delta(a, u, q[0]);
     }
     unsigned big = __ballot_sync(kFull, nw > 8u);
     while (big) {
@@ -719,19 +754,20 @@ __device__ __forceinline__ void finish_rows(const BcArgs &a, uint32_t s0, uint32
     }
 }
 
-template <int WT>
-__global__ void __launch_bounds__(kBcTPB, 1) bc_dag(BcArgs a) {
+// The passes of one source, by CTA `rank` of its nblocks.
+template <int WT, bool Word>
+__device__ __forceinline__ void dag_passes(const BcArgs &a, uint32_t rank, uint32_t nblocks) {
     __shared__ uint32_t s_pub[7];
     __shared__ uint32_t s_nw;
     __shared__ Stage st;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (a.nblocks * blockDim.x) >> 5;
+    const uint32_t gwarp = (rank * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (nblocks * blockDim.x) >> 5;
     uint32_t gen = 0;
     BcCtl *c = a.ctl;
-    // ---- COUNT (CTA 0 also puts the source on level 0)
+    // ---- COUNT (the group's first CTA also puts the source on level 0)
     if (threadIdx.x == 0) st.n = 0;
-    if (blockIdx.x == 0) {
+    if (rank == 0) {
         if (threadIdx.x == 0) {
             c->t0 = globaltimer();
             a.order[0] = a.source;
@@ -747,9 +783,12 @@ __global__ void __launch_bounds__(kBcTPB, 1) bc_dag(BcArgs a) {
         if (threadIdx.x < 32 && s_nw) fill_row(a, 0u, a.source, 0u, s_nw);
     }
     unsigned long long tight_n = 0;
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < a.n; u += a.nblocks * blockDim.x)
-        if (__ldg(a.dp + u) != kUnreached) a.sigma[u] = u == a.source ? 1ull : 0ull;
-    count_words<WT>(a, gwarp, nwarps, tight_n);
+    using S = State<WT, Word>;
+    for (uint32_t u = rank * blockDim.x + threadIdx.x; u < a.n; u += nblocks * blockDim.x) {
+        if (!a.bc) a.delta[u] = 0.0;   // k_bc_sum reads it; the source and unreached vertices keep it
+        if (__ldg(static_cast<const typename S::T *>(a.state) + u) != S::kNone) a.sigma[u] = u == a.source ? 1ull : 0ull;
+    }
+    count_words<WT, Word>(a, gwarp, nwarps, tight_n);
     for (int o = 16; o > 0; o >>= 1) tight_n += __shfl_down_sync(kFull, tight_n, o);
     if (lane == 0 && tight_n) atomicAdd(&a.tot->tight, tight_n);
     uint32_t L = 0;
@@ -789,7 +828,7 @@ __global__ void __launch_bounds__(kBcTPB, 1) bc_dag(BcArgs a) {
         ++L;
     }
     // L = number of levels; level k is order[lvl[k], lvl[k + 1])
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (rank == 0 && threadIdx.x == 0) {
         atomicMax(&a.tot->max_levels, L);
         atomicAdd(&a.tot->reached, (unsigned long long)s_pub[1]);
     }
@@ -818,20 +857,38 @@ __global__ void __launch_bounds__(kBcTPB, 1) bc_dag(BcArgs a) {
     }
 }
 
-// Batched shortest paths hand back plain distances (uint32 / float32 bits,
-// UINT32_MAX / +inf unreached); the DAG passes read state words.
-template <bool F32>
-__global__ void k_pack_dist(const uint32_t *__restrict__ dist, uint32_t n, unsigned long long *__restrict__ dp) {
-    const uint32_t unreached = F32 ? 0x7F800000u : 0xFFFFFFFFu;
+// One source on the whole grid (arguments in constant memory: 7 % faster than
+// through shared memory on an R-MAT 22).
+template <int WT, bool Word>
+__global__ void __launch_bounds__(kBcTPB, 1) bc_dag(BcArgs a) {
+    dag_passes<WT, Word>(a, blockIdx.x, a.nblocks);
+}
+
+// Several sources: CTAs [g nblocks, (g + 1) nblocks) run the one of groups[g].
+template <int WT, bool Word>
+__global__ void __launch_bounds__(kBcTPB, 1) bc_dag_groups(const BcArgs *__restrict__ groups, uint32_t nblocks) {
+    __shared__ BcArgs a;
+    if (threadIdx.x == 0) a = groups[blockIdx.x / nblocks];
+    __syncthreads();
+    dag_passes<WT, Word>(a, blockIdx.x % nblocks, nblocks);
+}
+
+// bc[v] += the dependencies of `count` sources on v, one after the other.
+__global__ void k_bc_sum(const double *__restrict__ delta, uint32_t n, uint32_t count, double *__restrict__ bc) {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint32_t d = dist[v];
-        dp[v] = d == unreached ? kUnreached : (unsigned long long)d << 32;
+        double x = bc[v];
+        for (uint32_t i = 0; i < count; ++i) x = __dadd_rn(x, delta[(size_t)i * n + v]);
+        bc[v] = x;
     }
 }
 
 constexpr uint32_t kBcBatch = 64;   // sources per batched shortest-path launch
 
 struct BcState {
+    // arrays of `groups` sources, group g's at g times its size
+    uint32_t groups = 0;
+    size_t n_long = 0, long_words = 0;
+    BcArgs *d_args = nullptr;
     unsigned long long *sigma = nullptr;
     double *delta = nullptr;
     uint32_t *indeg = nullptr;
@@ -857,10 +914,93 @@ struct BcState {
     int blocks = 0;
 };
 
-const void *bc_kernel(gbs_weight_type wt) {
-    return wt == GBS_WEIGHT_F64   ? (const void *)bc_dag<2>
-           : wt == GBS_WEIGHT_F32 ? (const void *)bc_dag<1>
-                                  : (const void *)bc_dag<0>;
+template <int WT, bool Word>
+const void *bc_kernel_of(bool groups) {
+    return groups ? (const void *)bc_dag_groups<WT, Word> : (const void *)bc_dag<WT, Word>;
+}
+const void *bc_kernel(gbs_weight_type wt, bool word, bool groups) {
+    if (wt == GBS_WEIGHT_F64) return bc_kernel_of<2, true>(groups);
+    if (wt == GBS_WEIGHT_F32) return word ? bc_kernel_of<1, true>(groups) : bc_kernel_of<1, false>(groups);
+    return word ? bc_kernel_of<0, true>(groups) : bc_kernel_of<0, false>(groups);
+}
+
+void free_groups(BcState *b) {
+    cudaFree(b->d_args);
+    cudaFree(b->sigma);
+    cudaFree(b->delta);
+    cudaFree(b->indeg);
+    cudaFree(b->order);
+    cudaFree(b->lvl);
+    cudaFree(b->wlv);
+    cudaFree(b->slv);
+    cudaFree(b->lr_u);
+    cudaFree(b->lr_b);
+    cudaFree(b->lr_n);
+    cudaFree(b->vw_u);
+    cudaFree(b->vw_w);
+    cudaFree(b->vw_rm);
+    cudaFree(b->vw_part);
+    cudaFree(b->mask);
+    cudaFree(b->ctl);
+    b->d_args = nullptr;
+    b->sigma = nullptr;
+    b->delta = b->vw_part = nullptr;
+    b->indeg = b->order = b->lvl = b->wlv = b->slv = b->lr_u = b->lr_b = b->lr_n = nullptr;
+    b->vw_u = b->vw_w = b->vw_rm = b->mask = nullptr;
+    b->ctl = nullptr;
+    b->groups = 0;
+}
+
+// Bytes of one source's arrays.
+size_t group_bytes(const gbs_graph *g, const BcState *b) {
+    return (size_t)g->n * 36 + b->n_long * 12 + b->long_words * 20 + b->mask_words * 4 + sizeof(BcCtl);
+}
+
+// Sources a launch runs at once, at most `want`: while the words their passes
+// gather (distance, path count, dependency, in-degree and lists, about 32 bytes
+// a vertex) fit in L2 together, and their arrays in a quarter of the free
+// memory.  Beyond L2 a source's big levels fill the GPU alone (R-MAT 22: one).
+uint32_t bc_groups(const gbs_graph *g, const BcState *b, uint32_t want) {
+    int l2 = 0;
+    size_t free_b = 0, total_b = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, g->device) != cudaSuccess ||
+        cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
+    const size_t fit = (size_t)l2 / (32 * (size_t)g->n);
+    const size_t mem = (free_b / 4 + b->groups * group_bytes(g, b)) / group_bytes(g, b);
+    const size_t most = std::min({(size_t)want, fit, mem, (size_t)b->blocks});
+    return (uint32_t)std::max<size_t>(most, 1);
+}
+
+// Arrays for `groups` sources (kept for later calls; they only grow).
+gbs_status ensure_groups(gbs_graph *g, BcState *b, uint32_t groups) {
+    if (b->groups >= groups) return GBS_OK;
+    free_groups(b);
+    const size_t n = g->n, G = groups;
+    const size_t lr = std::max<size_t>(b->n_long, 1), vw = std::max<size_t>(b->long_words, 1);
+    GBS_CUDA(cudaMalloc(&b->d_args, sizeof(BcArgs) * G));
+    GBS_CUDA(cudaMalloc(&b->sigma, sizeof(unsigned long long) * n * G));
+    GBS_CUDA(cudaMalloc(&b->delta, sizeof(double) * n * G));
+    GBS_CUDA(cudaMalloc(&b->indeg, sizeof(uint32_t) * n * G));
+    GBS_CUDA(cudaMalloc(&b->order, sizeof(uint32_t) * n * G));
+    GBS_CUDA(cudaMalloc(&b->lvl, sizeof(uint32_t) * (n + 1) * G));
+    GBS_CUDA(cudaMalloc(&b->wlv, sizeof(uint32_t) * (n + 1) * G));
+    GBS_CUDA(cudaMalloc(&b->slv, sizeof(uint32_t) * (n + 1) * G));
+    GBS_CUDA(cudaMalloc(&b->lr_u, sizeof(uint32_t) * lr * G));
+    GBS_CUDA(cudaMalloc(&b->lr_b, sizeof(uint32_t) * lr * G));
+    GBS_CUDA(cudaMalloc(&b->lr_n, sizeof(uint32_t) * lr * G));
+    GBS_CUDA(cudaMalloc(&b->vw_u, sizeof(uint32_t) * vw * G));
+    GBS_CUDA(cudaMalloc(&b->vw_w, sizeof(uint32_t) * vw * G));
+    GBS_CUDA(cudaMalloc(&b->vw_rm, sizeof(uint32_t) * vw * G));
+    GBS_CUDA(cudaMalloc(&b->vw_part, sizeof(double) * vw * G));
+    GBS_CUDA(cudaMalloc(&b->mask, sizeof(uint32_t) * b->mask_words * G));
+    GBS_CUDA(cudaMalloc(&b->ctl, sizeof(BcCtl) * G));
+    // in-degrees return to zero at the end of every FORWARD pass
+    GBS_CUDA(cudaMemsetAsync(b->indeg, 0, sizeof(uint32_t) * n * G, g->stream));
+    b->groups = groups;
+    return GBS_OK;
 }
 
 gbs_status alloc_bc(gbs_graph *g) {
@@ -893,35 +1033,23 @@ gbs_status alloc_bc(gbs_graph *g) {
     }
     b->n_words = n_words;
     b->mask_words = (size_t)(g->m >> 5) + 1;
-    GBS_CUDA(cudaMalloc(&b->sigma, sizeof(unsigned long long) * n));
-    GBS_CUDA(cudaMalloc(&b->delta, sizeof(double) * n));
-    GBS_CUDA(cudaMalloc(&b->indeg, sizeof(uint32_t) * n));
-    GBS_CUDA(cudaMalloc(&b->order, sizeof(uint32_t) * n));
-    GBS_CUDA(cudaMalloc(&b->lvl, sizeof(uint32_t) * (n + 1)));
-    GBS_CUDA(cudaMalloc(&b->wlv, sizeof(uint32_t) * (n + 1)));
-    GBS_CUDA(cudaMalloc(&b->lr_u, sizeof(uint32_t) * std::max<size_t>(n_long, 1)));
-    GBS_CUDA(cudaMalloc(&b->lr_b, sizeof(uint32_t) * std::max<size_t>(n_long, 1)));
-    GBS_CUDA(cudaMalloc(&b->slv, sizeof(uint32_t) * (n + 1)));
-    GBS_CUDA(cudaMalloc(&b->lr_n, sizeof(uint32_t) * std::max<size_t>(n_long, 1)));
-    GBS_CUDA(cudaMalloc(&b->vw_u, sizeof(uint32_t) * std::max<size_t>(long_words, 1)));
-    GBS_CUDA(cudaMalloc(&b->vw_w, sizeof(uint32_t) * std::max<size_t>(long_words, 1)));
-    GBS_CUDA(cudaMalloc(&b->vw_rm, sizeof(uint32_t) * std::max<size_t>(long_words, 1)));
-    GBS_CUDA(cudaMalloc(&b->vw_part, sizeof(double) * std::max<size_t>(long_words, 1)));
-    GBS_CUDA(cudaMalloc(&b->mask, sizeof(uint32_t) * b->mask_words));
+    b->n_long = n_long;
+    b->long_words = long_words;
     GBS_CUDA(cudaMalloc(&b->ne_rows, sizeof(uint32_t) * std::max<size_t>(ne_rows.size(), 1)));
     GBS_CUDA(cudaMalloc(&b->wown, sizeof(uint2) * wown.size()));
     if (!ne_rows.empty())
         GBS_CUDA(cudaMemcpy(b->ne_rows, ne_rows.data(), sizeof(uint32_t) * ne_rows.size(), cudaMemcpyHostToDevice));
     GBS_CUDA(cudaMemcpy(b->wown, wown.data(), sizeof(uint2) * wown.size(), cudaMemcpyHostToDevice));
     GBS_CUDA(cudaMalloc(&b->bc, sizeof(double) * n));
-    GBS_CUDA(cudaMalloc(&b->ctl, sizeof(BcCtl)));
     GBS_CUDA(cudaMalloc(&b->tot, sizeof(BcTotals)));
-    // in-degrees return to zero at the end of every FORWARD pass
-    GBS_CUDA(cudaMemsetAsync(b->indeg, 0, sizeof(uint32_t) * n, g->stream));
-    int per_sm = 0;
-    GBS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bc_kernel(g->wtype), kBcTPB, 0));
+    int per_sm = 1;
+    for (int q = 0; q < 4; ++q) {
+        int x = 0;
+        GBS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x, bc_kernel(g->wtype, q & 1, q & 2), kBcTPB, 0));
+        per_sm = std::min(per_sm, x);
+    }
     if (per_sm < 1) return fail(GBS_ERR_UNSUPPORTED, "betweenness kernel cannot be resident");
-    b->blocks = std::min(per_sm, 1) * g->sms;
+    b->blocks = per_sm * g->sms;
     return GBS_OK;
 }
 
@@ -930,25 +1058,10 @@ gbs_status alloc_bc(gbs_graph *g) {
 void free_bc(gbs_graph *g) {
     BcState *b = static_cast<BcState *>(g->bc);
     if (!b) return;
-    cudaFree(b->sigma);
-    cudaFree(b->delta);
-    cudaFree(b->indeg);
-    cudaFree(b->order);
-    cudaFree(b->lvl);
-    cudaFree(b->wlv);
-    cudaFree(b->lr_u);
-    cudaFree(b->lr_b);
-    cudaFree(b->slv);
-    cudaFree(b->lr_n);
-    cudaFree(b->vw_u);
-    cudaFree(b->vw_w);
-    cudaFree(b->vw_rm);
-    cudaFree(b->vw_part);
-    cudaFree(b->mask);
+    free_groups(b);
     cudaFree(b->ne_rows);
     cudaFree(b->wown);
     cudaFree(b->bc);
-    cudaFree(b->ctl);
     cudaFree(b->tot);
     delete b;
     g->bc = nullptr;
@@ -982,78 +1095,115 @@ gbs_status run_bc(gbs_graph *g, const uint32_t *sources, uint32_t k, const gbs_p
     GBS_CUDA(cudaMemsetAsync(b->tot, 0, sizeof(BcTotals), s));
     gbs_params p = params ? *params : gbs_params{};
     p.flags &= ~(uint32_t)(GBS_F_TRACE | GBS_F_FEATURES);
-    BcArgs a{};
-    a.row = g->d_row;
-    a.adj = g->d_adj;
-    a.w64 = g->d_w64;
-    a.dp = g->ws.dp;
-    a.n = g->n;
-    a.sigma = b->sigma;
-    a.delta = b->delta;
-    a.indeg = b->indeg;
-    a.order = b->order;
-    a.lvl = b->lvl;
-    a.wlv = b->wlv;
-    a.lr_u = b->lr_u;
-    a.lr_b = b->lr_b;
-    a.slv = b->slv;
-    a.lr_n = b->lr_n;
-    a.vw_u = b->vw_u;
-    a.vw_w = b->vw_w;
-    a.vw_rm = b->vw_rm;
-    a.vw_part = b->vw_part;
-    a.mask = b->mask;
-    a.ne_rows = b->ne_rows;
-    a.wown = b->wown;
-    a.n_words = b->n_words;
-    a.m = (uint32_t)g->m;
-    a.bc = bc_dev;
-    a.ctl = b->ctl;
-    a.tot = b->tot;
-    a.wait_ns = (unsigned long long)(p.wait_limit_ms ? p.wait_limit_ms : 4000u) * 1000000ull;
-    a.nblocks = (uint32_t)b->blocks;
     const bool want_trace = params && (params->flags & GBS_F_TRACE);
     if (want_trace) {
         if (!g->ws.trace) {
             g->ws.trace_cap = 1u << 20;
             GBS_CUDA(cudaMalloc(&g->ws.trace, sizeof(TraceRec) * g->ws.trace_cap));
         }
-        a.trace = g->ws.trace;
-        a.trace_cap = g->ws.trace_cap;
     }
-    const void *kfn = bc_kernel(g->wtype);
     gbs_bc_stats tot{};
     double dag_ms = 0.0;
-    // one DAG launch on the distances now in the workspace's state words
-    auto dag = [&](uint32_t src) -> gbs_status {
-        a.source = src;
-        void *args[] = {&a};
-        GBS_CUDA(cudaEventRecord(e0, s));
-        GBS_CUDA(cudaMemsetAsync(b->ctl, 0, sizeof(BcCtl), s));
-        GBS_CUDA(cudaMemsetAsync(b->mask, 0, sizeof(uint32_t) * b->mask_words, s));
-        GBS_CUDA(cudaLaunchCooperativeKernel(kfn, dim3(b->blocks), dim3(kBcTPB), args, 0, s));
-        GBS_CUDA(cudaEventRecord(e1, s));
-        GBS_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        GBS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        dag_ms += ms;
+    // the trace shows one source's passes on the whole grid
+    const uint32_t groups = want_trace ? 1u : bc_groups(g, b, k);
+    st = ensure_groups(g, b, groups);
+    std::vector<BcArgs> args(groups);
+    // the DAG passes of `cnt` sources, `groups` at a time: source i's distances
+    // are the n values at state + i * n of their type
+    auto dag = [&](const uint32_t *srcs, uint32_t cnt, const void *state, bool word) -> gbs_status {
+        const size_t n = g->n, lr = std::max<size_t>(b->n_long, 1), vw = std::max<size_t>(b->long_words, 1);
+        for (uint32_t i0 = 0; i0 < cnt; i0 += groups) {
+            const uint32_t here = std::min(groups, cnt - i0), ctas = (uint32_t)b->blocks / here;
+            for (uint32_t q = 0; q < here; ++q) {
+                BcArgs a{};
+                a.row = g->d_row;
+                a.adj = g->d_adj;
+                a.w64 = g->d_w64;
+                a.state = static_cast<const char *>(state) + (word ? 8 : 4) * n * (i0 + q);
+                a.n = g->n;
+                a.source = srcs[i0 + q];
+                a.sigma = b->sigma + n * q;
+                a.delta = b->delta + n * q;
+                a.indeg = b->indeg + n * q;
+                a.order = b->order + n * q;
+                a.lvl = b->lvl + (n + 1) * q;
+                a.wlv = b->wlv + (n + 1) * q;
+                a.slv = b->slv + (n + 1) * q;
+                a.mask = b->mask + b->mask_words * q;
+                a.lr_u = b->lr_u + lr * q;
+                a.lr_b = b->lr_b + lr * q;
+                a.lr_n = b->lr_n + lr * q;
+                a.vw_u = b->vw_u + vw * q;
+                a.vw_w = b->vw_w + vw * q;
+                a.vw_rm = b->vw_rm + vw * q;
+                a.vw_part = b->vw_part + vw * q;
+                a.ne_rows = b->ne_rows;
+                a.wown = b->wown;
+                a.n_words = b->n_words;
+                a.m = (uint32_t)g->m;
+                a.bc = groups == 1 ? bc_dev : nullptr;
+                a.ctl = b->ctl + q;
+                a.tot = b->tot;
+                if (want_trace) {
+                    a.trace = g->ws.trace;
+                    a.trace_cap = g->ws.trace_cap;
+                }
+                a.wait_ns = (unsigned long long)(p.wait_limit_ms ? p.wait_limit_ms : 4000u) * 1000000ull;
+                a.nblocks = ctas;
+                args[q] = a;
+            }
+            const BcArgs *d_args = b->d_args;
+            uint32_t nblocks = ctas;
+            void *many[] = {&d_args, &nblocks}, *one[] = {args.data()};
+            if (here > 1)
+                GBS_CUDA(cudaMemcpyAsync(b->d_args, args.data(), sizeof(BcArgs) * here, cudaMemcpyHostToDevice, s));
+            GBS_CUDA(cudaEventRecord(e0, s));
+            GBS_CUDA(cudaMemsetAsync(b->ctl, 0, sizeof(BcCtl) * here, s));
+            GBS_CUDA(cudaMemsetAsync(b->mask, 0, sizeof(uint32_t) * b->mask_words * here, s));
+            GBS_CUDA(cudaLaunchCooperativeKernel(bc_kernel(g->wtype, word, here > 1), dim3(ctas * here), dim3(kBcTPB),
+                                                 here > 1 ? many : one, 0, s));
+            if (groups > 1)
+                k_bc_sum<<<std::max(1, std::min<int>((g->n + 255) / 256, g->sms * 8)), 256, 0, s>>>(b->delta, g->n, here,
+                                                                                                    bc_dev);
+            GBS_CUDA(cudaGetLastError());
+            GBS_CUDA(cudaEventRecord(e1, s));
+            GBS_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            GBS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            dag_ms += ms;
+        }
         return GBS_OK;
     };
     const bool batched = g->wtype != GBS_WEIGHT_F64 && k > 1 &&
                          !(p.flags & (GBS_F_BC_SINGLE | GBS_F_LEARNED));
     if (!batched) {
-        for (uint32_t i = 0; i < k && st == GBS_OK; ++i) {
-            const uint32_t src = sources ? sources[i] : i;
-            gbs_stats one{};
-            st = run_sssp(g, src, &p, nullptr, nullptr, &one);
-            if (st != GBS_OK) break;
-            tot.sssp_ms += one.device_ms;
-            tot.edges_reached += one.edges_reached;
-            st = dag(src);
+        // one shortest-path run per source; the state words of several sources
+        // are set aside for a launch of as many groups
+        unsigned long long *words = nullptr;
+        if (st == GBS_OK && groups > 1 && cudaMalloc(&words, sizeof(unsigned long long) * groups * g->n) != cudaSuccess) {
+            cudaGetLastError();
+            st = fail(GBS_ERR_NO_MEMORY, "betweenness: no room for the state words");
         }
+        std::vector<uint32_t> cs(groups);
+        for (uint32_t i0 = 0; i0 < k && st == GBS_OK; i0 += groups) {
+            const uint32_t cnt = std::min(groups, k - i0);
+            for (uint32_t j = 0; j < cnt && st == GBS_OK; ++j) {
+                cs[j] = sources ? sources[i0 + j] : i0 + j;
+                gbs_stats one{};
+                st = run_sssp(g, cs[j], &p, nullptr, nullptr, &one);
+                if (st != GBS_OK) break;
+                tot.sssp_ms += one.device_ms;
+                tot.edges_reached += one.edges_reached;
+                if (words && cudaMemcpyAsync(words + (size_t)j * g->n, g->ws.dp, sizeof(unsigned long long) * g->n,
+                                             cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+                    st = fail(GBS_ERR_CUDA, "betweenness: copy failed");
+            }
+            if (st == GBS_OK) st = dag(cs.data(), cnt, words ? words : g->ws.dp, true);
+        }
+        cudaFree(words);
     } else {
         // up to kBcBatch sources per batched launch, distances kept on the
-        // device; each source's DAG passes then run on its distances
+        // device; the sources' DAG passes then run on them
         gbs_batch_params bp{};
         bp.delta = p.delta;
         bp.light = p.light;
@@ -1064,7 +1214,7 @@ gbs_status run_bc(gbs_graph *g, const uint32_t *sources, uint32_t k, const gbs_p
         bp.inline_edges = p.inline_edges;
         const uint32_t chunk = std::min(k, kBcBatch);
         uint32_t *bdist = nullptr;
-        if (cudaMalloc(&bdist, sizeof(uint32_t) * (size_t)chunk * g->n) != cudaSuccess) {
+        if (st == GBS_OK && cudaMalloc(&bdist, sizeof(uint32_t) * (size_t)chunk * g->n) != cudaSuccess) {
             cudaGetLastError();
             st = fail(GBS_ERR_NO_MEMORY, "betweenness: no room for the batched distances");
         }
@@ -1082,15 +1232,7 @@ gbs_status run_bc(gbs_graph *g, const uint32_t *sources, uint32_t k, const gbs_p
             if (st != GBS_OK) break;
             tot.sssp_ms += bs.device_ms;
             tot.edges_reached += bs.edges_reached;
-            const int tb = 256, eb = std::max(1, std::min<int>((g->n + tb - 1) / tb, g->sms * 8));
-            for (uint32_t j = 0; j < cnt && st == GBS_OK; ++j) {
-                if (g->wtype == GBS_WEIGHT_F32)
-                    k_pack_dist<true><<<eb, tb, 0, s>>>(bdist + (size_t)j * g->n, g->n, g->ws.dp);
-                else
-                    k_pack_dist<false><<<eb, tb, 0, s>>>(bdist + (size_t)j * g->n, g->n, g->ws.dp);
-                if (cudaGetLastError() != cudaSuccess) st = fail(GBS_ERR_CUDA, "betweenness: launch failed");
-                else st = dag(cs[j]);
-            }
+            st = dag(cs.data(), cnt, bdist, false);
         }
         cudaFree(bdist);
     }

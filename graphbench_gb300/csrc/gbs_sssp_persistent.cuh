@@ -670,7 +670,10 @@ __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const
             }
             wide = max(wide, (uint32_t)__popc(__ballot_sync(FULL, lane < kMergeLow && incl <= a.merge_low)));
         }
-        span = max(span, wide);
+        if (wide > span) {
+            span = wide;
+            if (a.ctrl == kCtrlFixed) full = 1u;
+        }
     }
     // a bucket never reaches past the smallest pending bucket
     while (span > 1u && pend > 0u && nb + span > pm) span >>= 1;
