@@ -261,6 +261,7 @@ struct SsspArgs {
     uint32_t merge_low;     // a bucket takes in the next base buckets while their lists hold at most
                             // this many entries (0: no such merge; see merge_spans)
     uint32_t merge_drain;   // base buckets a bucket takes in while the run drains (0 or 1: none)
+    uint32_t merge_whole;   // 1: merged buckets relax whole rows whatever full_items says
     // bucket-width controller
     uint32_t ctrl;          // CtrlMode
     uint32_t span_fixed;    // kCtrlFixed: base widths per bucket (0 or 1 = plain delta-stepping)

@@ -672,7 +672,7 @@ __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const
         }
         if (wide > span) {
             span = wide;
-            if (a.ctrl == kCtrlFixed) full = 1u;
+            if (a.merge_whole) full = 1u;
         }
     }
     // a bucket never reaches past the smallest pending bucket
