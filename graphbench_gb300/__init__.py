@@ -721,7 +721,9 @@ def _tcsr_to_graph(gs: TCsr) -> Graph:
     row = np.zeros(len(ends) + 1, dtype=np.uint64)
     row[1:] = ends
     w = np.asarray(gs.edge_weight, dtype=np.float64)
-    if np.all(w == np.floor(w)) and (len(w) == 0 or (w.min() >= 0 and w.max() < 2**32 - 1)):
+    # fractional weights nearly always show in the first entries: the pass over
+    # all of them is for the others
+    if all(np.all(x == np.floor(x)) for x in (w[:4096], w)) and (len(w) == 0 or (w.min() >= 0 and w.max() < 2**32 - 1)):
         return Graph(row, gs.edge_idx, w.astype(np.uint32))
     return Graph(row, gs.edge_idx, w)
 

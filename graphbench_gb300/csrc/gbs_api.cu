@@ -208,17 +208,24 @@ void sort_rows64(const uint64_t *row, const uint32_t *cols, const uint64_t *wbit
     for (auto &t : th) t.join();
 }
 
-gbs_status prepare_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, const uint32_t *cols,
-                       const void *weights, gbs_weight_type wtype, std::vector<uint32_t> &row32,
-                       std::vector<uint2> &adj, double &max_w, std::vector<unsigned long long> *w64) {
+gbs_status check_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, const uint32_t *cols, const void *weights,
+                     gbs_weight_type wtype, bool f64) {
     if (!row_offsets || (m && (!cols || !weights)))
         return fail(GBS_ERR_INVALID_ARG, "NULL CSR array");
-    if (wtype != GBS_WEIGHT_U32 && wtype != GBS_WEIGHT_F32 && !(wtype == GBS_WEIGHT_F64 && w64))
+    if (wtype != GBS_WEIGHT_U32 && wtype != GBS_WEIGHT_F32 && !(wtype == GBS_WEIGHT_F64 && f64))
         return fail(GBS_ERR_INVALID_ARG, "unknown or unsupported weight type");
     if (n == 0 || n > 0x7FFFFFFFu) return fail(GBS_ERR_INVALID_ARG, "vertex count must be in [1, 2^31)");
     if (m >= 0xFFFFFFFFull) return fail(GBS_ERR_UNSUPPORTED, "edge count must be < 2^32");
     if (row_offsets[0] != 0 || row_offsets[n] != m)
         return fail(GBS_ERR_INVALID_ARG, "row_offsets must start at 0 and end at m");
+    return GBS_OK;
+}
+
+gbs_status prepare_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, const uint32_t *cols,
+                       const void *weights, gbs_weight_type wtype, std::vector<uint32_t> &row32,
+                       std::vector<uint2> &adj, double &max_w, std::vector<unsigned long long> *w64) {
+    const gbs_status st = check_csr(n, m, row_offsets, cols, weights, wtype, w64 != nullptr);
+    if (st != GBS_OK) return st;
     for (uint32_t v = 0; v < n; ++v)
         if (row_offsets[v + 1] < row_offsets[v]) return fail(GBS_ERR_INVALID_ARG, "row_offsets decrease");
     max_w = 0.0;
@@ -785,11 +792,17 @@ gbs_status gbs_graph_create(uint32_t n, uint64_t m, const uint64_t *row_offsets,
                             const void *weights, gbs_weight_type wtype, gbs_graph **out) {
     if (!out) return fail(GBS_ERR_INVALID_ARG, "out is NULL");
     *out = nullptr;
+    gbs_status st = check_csr(n, m, row_offsets, cols, weights, wtype, true);
+    if (st != GBS_OK) return st;
+    // checked and sorted on the device; on the host where its arrays do not
+    // fit beside the graph
+    st = graph_from_host(n, m, row_offsets, cols, weights, wtype, out);
+    if (st != GBS_ERR_NO_MEMORY) return st;
     std::vector<uint32_t> row32;
     std::vector<uint2> adj;
     double max_w = 0.0;
     std::vector<unsigned long long> w64;
-    gbs_status st = prepare_csr(n, m, row_offsets, cols, weights, wtype, row32, adj, max_w, &w64);
+    st = prepare_csr(n, m, row_offsets, cols, weights, wtype, row32, adj, max_w, &w64);
     if (st != GBS_OK) return st;
     double wsum = 0.0;
     for (uint64_t e = 0; e < m; ++e)

@@ -110,6 +110,8 @@ void sort_rows(const uint64_t *row, const uint32_t *cols, const uint32_t *wbits,
 // float32, -0 stored as +0) and returns its uint32 offsets, its rows sorted
 // by (weight, col) as {col, weight bits} and its largest weight.
 // float64 weights (w64 given) keep adj = {col, 0} and the weights in w64.
+gbs_status check_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, const uint32_t *cols, const void *weights,
+                     gbs_weight_type wtype, bool f64);   // the checks that need no pass over the arrays
 gbs_status prepare_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, const uint32_t *cols,
                        const void *weights, gbs_weight_type wtype, std::vector<uint32_t> &row32,
                        std::vector<uint2> &adj, double &max_w, std::vector<unsigned long long> *w64 = nullptr);
@@ -133,6 +135,13 @@ int persistent_ctas_per_sm(gbs_weight_type wt, bool batch);
 gbs_status graph_shell(uint32_t n, uint64_t m, gbs_weight_type wtype, double max_w, double mean_w, bool zero_w,
                        gbs_graph **out);
 void free_graph(gbs_graph *g);
+
+// A resident graph from host arrays, checked and sorted on the device
+// (gbs_ingest.cu).  The caller has checked the pointers, n, m and the first and
+// last row offset.  It holds up to 92 bytes per edge beside the graph while it
+// runs (GBS_ERR_NO_MEMORY where they are not there).
+gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const uint32_t *cols, const void *weights,
+                           gbs_weight_type wtype, gbs_graph **out);
 
 // Allocates the single-source workspace of a graph on first use.
 gbs_status ensure_workspace(gbs_graph *g);

@@ -32,6 +32,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <chrono>
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -223,50 +224,103 @@ __global__ void k_split(const long long *__restrict__ pairs, unsigned long long 
 }
 
 // ------------------------------------------------- resident graph build
-__global__ void k_row_of(const unsigned long long *__restrict__ row, uint32_t n, uint32_t *__restrict__ row_of) {
-    const unsigned lane = threadIdx.x & 31u;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += warps)
-        for (unsigned long long e = row[v] + lane; e < row[v + 1]; e += 32ull) row_of[e] = v;
-}
+// What the pass over the edges finds.
+struct EdgeStats {
+    unsigned long long bad;       // 4 x the first bad edge + what is wrong (kBad*); ~0: none
+    unsigned long long max_bits;  // largest weight, bits of its type
+    double sum;                   // of the weights
+    uint32_t unsorted;            // a row's columns are not in ascending order
+    uint32_t zero;                // a weight is zero
+    uint32_t rows_bad;            // row offsets decrease
+    uint32_t max_deg;             // longest row
+};
+enum : uint32_t { kBadCol = 0, kBadWeight = 1, kBadInteger = 2 };
 
-// Weight bits of the resident graph; flags bit 0: a weight is negative or not
-// finite, bit 1: not an integer in [0, 2^32) (uint32 graphs), bit 2: zero.
-template <int WT>
-__global__ void k_weight_bits(const double *__restrict__ w, unsigned long long m, unsigned long long *__restrict__ bits,
-                              uint32_t *flags) {
-    uint32_t f = 0;
-    for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; e < m;
-         e += (unsigned long long)gridDim.x * blockDim.x) {
-        double x = w[e];
-        if (!(x >= 0.0) || isinf(x)) {
-            f |= 1u;
-            x = 0.0;
+// Weight bits of type WT (0 uint32, 1 float32, 2 float64) from a source of the
+// same type or from a device CSR's doubles; -0 as +0.  Returns kBad* or ~0u.
+template <int WT, typename Src>
+__device__ __forceinline__ uint32_t weight_bits(Src w, unsigned long long &bits) {
+    if constexpr (sizeof(Src) == 4 && WT == 0) {
+        bits = w;
+        return ~0u;
+    } else {
+        if (!(w >= Src(0)) || isinf(w)) {
+            bits = 0ull;
+            return kBadWeight;
         }
-        if (x == 0.0) {
-            f |= 4u;
-            x = 0.0;   // -0 as +0
-        }
-        if (WT == 2) {
-            bits[e] = (unsigned long long)__double_as_longlong(x);
-        } else if (WT == 1) {
-            bits[e] = __float_as_uint(__double2float_rn(x));
+        if (w == Src(0)) w = Src(0);
+        if constexpr (WT == 2) {
+            bits = (unsigned long long)__double_as_longlong(w);
+        } else if constexpr (WT == 1) {
+            bits = __float_as_uint((float)w);
         } else {
-            if (x != floor(x) || x > 4294967295.0) f |= 2u;
-            bits[e] = (unsigned long long)(uint32_t)x;
+            bits = (unsigned long long)(uint32_t)w;
+            if (w != floor(w) || w > Src(4294967295.0)) return kBadInteger;
         }
+        return ~0u;
     }
-    if (f) atomicOr(flags, f);
 }
 
-__global__ void k_key_row_w(const uint32_t *__restrict__ row_of, const unsigned long long *__restrict__ wbits,
-                            const uint32_t *__restrict__ id, unsigned long long m, unsigned long long *__restrict__ key) {
-    for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
-         p += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t e = id[p];
-        key[p] = ((unsigned long long)row_of[e] << 32) | wbits[e];
+// One pass over the edges in CSR order: every edge's row, checks, the sort key
+// (uint32 / float32: row << 32 | weight bits; float64: weight bits, the row
+// beside it) and the statistics.  A warp takes 1,024 consecutive edges, a lane
+// every 32nd of them: its row is found by a search once and then by walking on.
+// A search stays inside the offsets even where they decrease (the caller looks
+// at rows_bad first).
+constexpr uint32_t kEdgeTile = 1024;
+template <int WT, typename Src>
+__global__ void __launch_bounds__(256) k_edges(const unsigned long long *__restrict__ row, const uint32_t *__restrict__ col,
+                                               const Src *__restrict__ w, uint32_t n, unsigned long long m,
+                                               unsigned long long *__restrict__ key, uint32_t *__restrict__ row_of,
+                                               EdgeStats *st) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
+    const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    unsigned long long mx = 0ull, bad = ~0ull;
+    double sum = 0.0;
+    bool unsorted = false, zero = false;
+    for (unsigned long long t = warp * kEdgeTile; t < m; t += warps * kEdgeTile) {
+        uint32_t v = 0, top = n - 1u;   // the last row that starts at or before the lane's first edge
+        while (v < top) {
+            const uint32_t mid = v + (top - v + 1u) / 2u;
+            if (row[mid] <= t + lane) v = mid;
+            else top = mid - 1u;
+        }
+        for (unsigned long long e = t + lane; e < min(m, t + kEdgeTile); e += 32u) {
+            while (v + 1u < n && row[v + 1u] <= e) ++v;
+            const uint32_t c = col[e];
+            unsigned long long bits;
+            const Src x = w[e];
+            const uint32_t why = weight_bits<WT, Src>(x, bits);
+            if (c >= n) bad = min(bad, 4ull * e + kBadCol);
+            else if (why != ~0u) bad = min(bad, 4ull * e + why);
+            unsorted |= e > row[v] && col[e - 1u] > c;
+            zero |= bits == 0ull;
+            mx = max(mx, bits);
+            sum += (double)x;
+            if (WT == 2) {
+                key[e] = bits;
+                row_of[e] = v;
+            } else {
+                key[e] = ((unsigned long long)v << 32) | bits;
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = max(mx, __shfl_down_sync(0xffffffffu, mx, o));
+        bad = min(bad, __shfl_down_sync(0xffffffffu, bad, o));
+        sum += __shfl_down_sync(0xffffffffu, sum, o);
+    }
+    if (__any_sync(0xffffffffu, unsorted) && lane == 0) st->unsorted = 1u;
+    if (__any_sync(0xffffffffu, zero) && lane == 0) st->zero = 1u;
+    if (lane == 0) {
+        if (mx) atomicMax(&st->max_bits, mx);
+        if (bad != ~0ull) atomicMin(&st->bad, bad);
+        if (sum != 0.0) atomicAdd(&st->sum, sum);
     }
 }
+
+__global__ void k_edge_stats_init(EdgeStats *st) { *st = EdgeStats{~0ull, 0ull, 0.0, 0u, 0u, 0u, 0u}; }
 
 template <typename K>
 __global__ void k_gather_key(const K *__restrict__ src, const uint32_t *__restrict__ id, unsigned long long m,
@@ -276,27 +330,40 @@ __global__ void k_gather_key(const K *__restrict__ src, const uint32_t *__restri
         key[p] = src[id[p]];
 }
 
-__global__ void k_adj(const uint32_t *__restrict__ id, const uint32_t *__restrict__ col,
-                      const unsigned long long *__restrict__ wbits, unsigned long long m, bool f64, uint2 *__restrict__ adj,
-                      unsigned long long *__restrict__ w64) {
+// Sorted (row, weight) keys and the columns that came with them.
+__global__ void k_adj32(const unsigned long long *__restrict__ key, const uint32_t *__restrict__ col,
+                        unsigned long long m, uint2 *__restrict__ adj) {
+    for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
+         p += (unsigned long long)gridDim.x * blockDim.x)
+        adj[p] = make_uint2(col[p], (uint32_t)key[p]);
+}
+
+__global__ void k_adj64(const uint32_t *__restrict__ id, const uint32_t *__restrict__ col,
+                        const unsigned long long *__restrict__ wbits, unsigned long long m, uint2 *__restrict__ adj,
+                        unsigned long long *__restrict__ w64) {
     for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
          p += (unsigned long long)gridDim.x * blockDim.x) {
         const uint32_t e = id[p];
-        adj[p] = make_uint2(col[e], f64 ? 0u : (uint32_t)wbits[e]);
-        if (f64) w64[p] = wbits[e];
+        adj[p] = make_uint2(col[e], 0u);
+        w64[p] = wbits[e];
     }
 }
 
-// max_deg: raised to the longest row
+// uint32 offsets, whether the offsets decrease, the longest row.
 __global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, uint32_t *__restrict__ row32,
-                        uint32_t *max_deg) {
+                        EdgeStats *st) {
     uint32_t d = 0;
+    bool bad = false;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
         row32[v] = (uint32_t)row[v];
-        if (v < n) d = max(d, (uint32_t)(row[v + 1] - row[v]));
+        if (v < n) {
+            d = max(d, (uint32_t)(row[v + 1] - row[v]));
+            bad |= row[v + 1] < row[v];
+        }
     }
     d = __reduce_max_sync(0xffffffffu, d);
-    if ((threadIdx.x & 31u) == 0) atomicMax(max_deg, d);
+    if ((threadIdx.x & 31u) == 0) atomicMax(&st->max_deg, d);
+    if (bad) st->rows_bad = 1u;
 }
 
 // ----------------------------------------------------------------- host
@@ -684,109 +751,163 @@ __global__ void k_iota(uint32_t *__restrict__ id, unsigned long long m) {
         id[k] = (uint32_t)k;
 }
 
-// A resident graph from a device CSR: rows sorted by (weight, column) with
-// stable radix passes from the least significant key up.
-gbs_status graph_from_csr(const gbs_device_csr *c, gbs_weight_type wtype, gbs_graph **out) {
-    if (wtype != GBS_WEIGHT_U32 && wtype != GBS_WEIGHT_F32 && wtype != GBS_WEIGHT_F64)
-        return fail(GBS_ERR_INVALID_ARG, "unknown weight type");
-    const unsigned long long m = c->m;
-    const uint32_t n = c->n;
-    int dev = 0, sms = 0;
-    ING_CUDA(cudaGetDevice(&dev));
-    ING_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    cudaStream_t s;
-    ING_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    struct StreamFree {
-        cudaStream_t s;
-        ~StreamFree() { cudaStreamDestroy(s); }
-    } sf{s};
-    Bufs bufs;
+// A resident graph from device arrays: rows sorted by (weight, column) with
+// stable radix passes, the columns first where some row does not have them in
+// ascending order.  `host`: the arrays come from gbs_graph_create (its
+// messages); else from a device CSR.  gbs_graph_create, checked and sorted by 16
+// host cores -> here, ms: R-MAT 16 6.5 -> 1.1 (float64 10.8 -> 1.7), 20 116 ->
+// 5.6, 22 475 -> 20.
+template <int WT, typename Src>
+gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long long *row, const uint32_t *col, const Src *w,
+                       bool host, int sms, cudaStream_t s, Bufs &bufs, gbs_graph **out) {
+    constexpr gbs_weight_type wtype = WT == 2 ? GBS_WEIGHT_F64 : WT == 1 ? GBS_WEIGHT_F32 : GBS_WEIGHT_U32;
+    constexpr bool f64 = WT == 2;
     const int gb = grid_for(m, sms);
-    uint32_t *row_of = nullptr, *flags = nullptr, *id0 = nullptr, *id1 = nullptr, *col_s = nullptr;
-    unsigned long long *wbits = nullptr, *key = nullptr, *key_s = nullptr;
-    ING_CUDA(bufs.get(&row_of, m));
-    ING_CUDA(bufs.get(&flags, 2));   // weight flags, longest row
-    ING_CUDA(bufs.get(&wbits, m));
-    ING_CUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(uint32_t), s));
-    k_row_of<<<std::max(1, std::min<int>((n + 7) / 8, sms * 16)), 256, 0, s>>>(c->d_row, n, row_of);
-    ING_CUDA(cudaGetLastError());
-    if (wtype == GBS_WEIGHT_F64) k_weight_bits<2><<<gb, 256, 0, s>>>(c->d_w, m, wbits, flags);
-    else if (wtype == GBS_WEIGHT_F32) k_weight_bits<1><<<gb, 256, 0, s>>>(c->d_w, m, wbits, flags);
-    else k_weight_bits<0><<<gb, 256, 0, s>>>(c->d_w, m, wbits, flags);
-    ING_CUDA(cudaGetLastError());
-    uint32_t hf = 0;
-    ING_CUDA(cudaMemcpyAsync(&hf, flags, sizeof(hf), cudaMemcpyDeviceToHost, s));
-    ING_CUDA(cudaStreamSynchronize(s));
-    if (hf & 1u) return fail(GBS_ERR_INVALID_ARG, "weights must be finite and >= 0");
-    if (hf & 2u) return fail(GBS_ERR_INVALID_ARG, "uint32 graphs need integer weights below 2^32");
-    // pass 1: by column
-    ING_CUDA(bufs.get(&id0, m));
-    ING_CUDA(bufs.get(&id1, m));
-    ING_CUDA(bufs.get(&col_s, m));
-    k_iota<<<gb, 256, 0, s>>>(id0, m);
-    ING_CUDA(cudaGetLastError());
-    gbs_status st = sort_pairs<uint32_t>(c->d_col, col_s, id0, id1, m, s, bufs);
-    if (st != GBS_OK) return st;
+    EdgeStats *st = nullptr, hs{};
+    unsigned long long *key = nullptr, *key_s = nullptr;
+    uint32_t *row_of = nullptr, *row32 = nullptr;
+    ING_CUDA(bufs.get(&st, 1));
     ING_CUDA(bufs.get(&key, m));
     ING_CUDA(bufs.get(&key_s, m));
-    if (wtype == GBS_WEIGHT_F64) {
-        // pass 2: by weight bits; pass 3: by row
-        k_gather_key<unsigned long long><<<gb, 256, 0, s>>>(wbits, id1, m, key);
-        ING_CUDA(cudaGetLastError());
-        st = sort_pairs<unsigned long long>(key, key_s, id1, id0, m, s, bufs);
-        if (st != GBS_OK) return st;
-        uint32_t *rk = reinterpret_cast<uint32_t *>(key), *rk_s = reinterpret_cast<uint32_t *>(key_s);
-        k_gather_key<uint32_t><<<gb, 256, 0, s>>>(row_of, id0, m, rk);
-        ING_CUDA(cudaGetLastError());
-        st = sort_pairs<uint32_t>(rk, rk_s, id0, id1, m, s, bufs);
-        if (st != GBS_OK) return st;
-    } else {
-        // pass 2: by (row, weight bits)
-        k_key_row_w<<<gb, 256, 0, s>>>(row_of, wbits, id1, m, key);
-        ING_CUDA(cudaGetLastError());
-        st = sort_pairs<unsigned long long>(key, key_s, id1, id0, m, s, bufs);
-        if (st != GBS_OK) return st;
-        std::swap(id0, id1);
+    if (f64) ING_CUDA(bufs.get(&row_of, m));
+    ING_CUDA(cudaMalloc(&row32, sizeof(uint32_t) * ((size_t)n + 1)));
+    struct Guard {   // row32 becomes the graph's; until then it is freed here
+        uint32_t *p;
+        ~Guard() { cudaFree(p); }
+    } guard{row32};
+    k_edge_stats_init<<<1, 1, 0, s>>>(st);
+    k_row32<<<std::max(1, std::min<int>((int)(((unsigned long long)n + 256) / 256), sms * 8)), 256, 0, s>>>(row, n, row32, st);
+    k_edges<WT, Src><<<grid_for((m + kEdgeTile - 1) / kEdgeTile * 32, sms), 256, 0, s>>>(row, col, w, n, m, key, row_of, st);
+    ING_CUDA(cudaGetLastError());
+    ING_CUDA(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s));
+    ING_CUDA(cudaStreamSynchronize(s));
+    if (hs.rows_bad) return fail(GBS_ERR_INVALID_ARG, "row_offsets decrease");
+    if (hs.bad != ~0ull) {
+        const uint32_t why = (uint32_t)(hs.bad & 3ull);
+        if (why == kBadCol) return fail(GBS_ERR_INVALID_ARG, "column index out of range");
+        if (why == kBadInteger) return fail(GBS_ERR_INVALID_ARG, "uint32 graphs need integer weights below 2^32");
+        return fail(GBS_ERR_INVALID_ARG, !host ? "weights must be finite and >= 0"
+                                         : f64 ? "float64 weights must be finite and >= 0"
+                                               : "float32 weights must be finite and >= 0");
     }
-    // id1: the edge at each sorted position
-    double hmax = 0.0, hsum = 0.0;
-    double *dred = nullptr;
-    ING_CUDA(bufs.get(&dred, 2));
-    {
-        size_t t1 = 0, t2 = 0;
-        ING_CUDA(cub::DeviceReduce::Max(nullptr, t1, c->d_w, dred, (int64_t)m, s));
-        ING_CUDA(cub::DeviceReduce::Sum(nullptr, t2, c->d_w, dred + 1, (int64_t)m, s));
-        char *t = nullptr;
-        ING_CUDA(bufs.get(&t, std::max(t1, t2)));
-        if (m) {
-            ING_CUDA(cub::DeviceReduce::Max(t, t1, c->d_w, dred, (int64_t)m, s));
-            ING_CUDA(cub::DeviceReduce::Sum(t, t2, c->d_w, dred + 1, (int64_t)m, s));
-            ING_CUDA(cudaMemcpyAsync(&hmax, dred, sizeof(double), cudaMemcpyDeviceToHost, s));
-            ING_CUDA(cudaMemcpyAsync(&hsum, dred + 1, sizeof(double), cudaMemcpyDeviceToHost, s));
+    double max_w = 0.0;
+    if (WT == 0) {
+        max_w = (double)hs.max_bits;
+    } else if (WT == 1) {
+        const uint32_t bits = (uint32_t)hs.max_bits;
+        float f;
+        std::memcpy(&f, &bits, 4);
+        max_w = f;
+    } else {
+        std::memcpy(&max_w, &hs.max_bits, 8);
+    }
+    int bits_n = 1;
+    while (bits_n < 32 && (1ull << bits_n) < n) ++bits_n;
+    // columns into order first, if they are not: id then lists the edges
+    uint32_t *id0 = nullptr, *id1 = nullptr, *col_s = nullptr;
+    const uint32_t *cols = col;   // the columns in the order of the keys
+    gbs_status r;
+    ING_CUDA(bufs.get(&col_s, m));
+    if (f64 || hs.unsorted) {
+        ING_CUDA(bufs.get(&id0, m));
+        ING_CUDA(bufs.get(&id1, m));
+        k_iota<<<gb, 256, 0, s>>>(id0, m);
+        ING_CUDA(cudaGetLastError());
+    }
+    if (hs.unsorted) {
+        if ((r = sort_pairs<uint32_t>(col, col_s, id0, id1, m, s, bufs, bits_n)) != GBS_OK) return r;
+        std::swap(id0, id1);
+        k_gather_key<unsigned long long><<<gb, 256, 0, s>>>(key, id0, m, key_s);
+        ING_CUDA(cudaGetLastError());
+        if (!f64) {
+            std::swap(key, key_s);
+            cols = col_s;
         }
     }
     gbs_graph *g = nullptr;
-    ING_CUDA(cudaStreamSynchronize(s));
-    const double max_w = wtype == GBS_WEIGHT_F32 ? (double)(float)hmax : hmax;
-    st = graph_shell(n, m, wtype, max_w, m ? hsum / (double)m : 0.0, (hf & 4u) != 0u, &g);
-    if (st != GBS_OK) return st;
-    cudaError_t e;
-    if ((e = cudaMalloc(&g->d_row, sizeof(uint32_t) * ((size_t)n + 1))) != cudaSuccess ||
-        (e = cudaMalloc(&g->d_adj, sizeof(uint2) * (m ? m : 1))) != cudaSuccess ||
-        (wtype == GBS_WEIGHT_F64 && (e = cudaMalloc(&g->d_w64, sizeof(unsigned long long) * (m ? m : 1))) != cudaSuccess)) {
+    if (f64) {
+        // by weight, then by row; key keeps the weights in edge order
+        unsigned long long *a = nullptr, *b = nullptr;
+        ING_CUDA(bufs.get(&a, m));
+        ING_CUDA(bufs.get(&b, m));
+        if ((r = sort_pairs<unsigned long long>(hs.unsorted ? key_s : key, a, id0, id1, m, s, bufs)) != GBS_OK) return r;
+        uint32_t *rk = reinterpret_cast<uint32_t *>(a), *rk_s = reinterpret_cast<uint32_t *>(b);
+        k_gather_key<uint32_t><<<gb, 256, 0, s>>>(row_of, id1, m, rk);
+        ING_CUDA(cudaGetLastError());
+        if ((r = sort_pairs<uint32_t>(rk, rk_s, id1, id0, m, s, bufs, bits_n)) != GBS_OK) return r;
+    } else {
+        uint32_t *c_out = cols == col_s ? nullptr : col_s;
+        if (!c_out) ING_CUDA(bufs.get(&c_out, m));
+        if ((r = sort_pairs<unsigned long long>(key, key_s, cols, c_out, m, s, bufs, 32 + bits_n)) != GBS_OK) return r;
+        cols = c_out;
+    }
+    if ((r = graph_shell(n, m, wtype, max_w, m ? hs.sum / (double)m : 0.0, hs.zero != 0u, &g)) != GBS_OK) return r;
+    cudaError_t e = cudaMalloc(&g->d_adj, sizeof(uint2) * (m ? m : 1));
+    if (e == cudaSuccess && f64) e = cudaMalloc(&g->d_w64, sizeof(unsigned long long) * (m ? m : 1));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
         free_graph(g);
         return fail(e == cudaErrorMemoryAllocation ? GBS_ERR_NO_MEMORY : GBS_ERR_CUDA, cudaGetErrorString(e));
     }
-    k_row32<<<std::max(1, std::min<int>((n + 256) / 256, sms * 8)), 256, 0, s>>>(c->d_row, n, g->d_row, flags + 1);
-    k_adj<<<gb, 256, 0, s>>>(id1, c->d_col, wbits, m, wtype == GBS_WEIGHT_F64, g->d_adj, g->d_w64);
-    if ((e = cudaGetLastError()) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&g->max_deg, flags + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess) {
+    if (f64) k_adj64<<<gb, 256, 0, s>>>(id0, col, key, m, g->d_adj, g->d_w64);
+    else k_adj32<<<gb, 256, 0, s>>>(key_s, cols, m, g->d_adj);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess) {
         free_graph(g);
         return fail(GBS_ERR_CUDA, cudaGetErrorString(e));
     }
+    g->d_row = row32;
+    guard.p = nullptr;
+    g->max_deg = hs.max_deg;
     *out = g;
     return GBS_OK;
+}
+
+struct StreamOf {
+    cudaStream_t s = nullptr;
+    ~StreamOf() {
+        if (s) cudaStreamDestroy(s);
+    }
+};
+
+gbs_status graph_from_csr(const gbs_device_csr *c, gbs_weight_type wtype, gbs_graph **out) {
+    if (wtype != GBS_WEIGHT_U32 && wtype != GBS_WEIGHT_F32 && wtype != GBS_WEIGHT_F64)
+        return fail(GBS_ERR_INVALID_ARG, "unknown weight type");
+    int dev = 0, sms = 0;
+    ING_CUDA(cudaGetDevice(&dev));
+    ING_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    StreamOf so;
+    ING_CUDA(cudaStreamCreateWithFlags(&so.s, cudaStreamNonBlocking));
+    Bufs bufs;
+    if (wtype == GBS_WEIGHT_F64) return build_graph<2, double>(c->n, c->m, c->d_row, c->d_col, c->d_w, false, sms, so.s, bufs, out);
+    if (wtype == GBS_WEIGHT_F32) return build_graph<1, double>(c->n, c->m, c->d_row, c->d_col, c->d_w, false, sms, so.s, bufs, out);
+    return build_graph<0, double>(c->n, c->m, c->d_row, c->d_col, c->d_w, false, sms, so.s, bufs, out);
+}
+
+gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const uint32_t *cols, const void *weights,
+                           gbs_weight_type wtype, gbs_graph **out) {
+    int dev = 0, sms = 0;
+    ING_CUDA(cudaGetDevice(&dev));
+    ING_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    StreamOf so;
+    ING_CUDA(cudaStreamCreateWithFlags(&so.s, cudaStreamNonBlocking));
+    Bufs bufs;
+    const size_t wb = dist_bytes(wtype);
+    unsigned long long *d_row = nullptr;
+    uint32_t *d_col = nullptr;
+    char *d_w = nullptr;
+    ING_CUDA(bufs.get(&d_row, (size_t)n + 1));
+    ING_CUDA(bufs.get(&d_col, m));
+    ING_CUDA(bufs.get(&d_w, wb * m));
+    ING_CUDA(cudaMemcpyAsync(d_row, row, 8ull * ((size_t)n + 1), cudaMemcpyHostToDevice, so.s));
+    if (m) {
+        ING_CUDA(cudaMemcpyAsync(d_col, cols, 4ull * m, cudaMemcpyHostToDevice, so.s));
+        ING_CUDA(cudaMemcpyAsync(d_w, weights, wb * m, cudaMemcpyHostToDevice, so.s));
+    }
+    if (wtype == GBS_WEIGHT_F64)
+        return build_graph<2, double>(n, m, d_row, d_col, reinterpret_cast<double *>(d_w), true, sms, so.s, bufs, out);
+    if (wtype == GBS_WEIGHT_F32)
+        return build_graph<1, float>(n, m, d_row, d_col, reinterpret_cast<float *>(d_w), true, sms, so.s, bufs, out);
+    return build_graph<0, uint32_t>(n, m, d_row, d_col, reinterpret_cast<uint32_t *>(d_w), true, sms, so.s, bufs, out);
 }
 
 }  // namespace gbs
