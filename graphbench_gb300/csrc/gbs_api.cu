@@ -15,6 +15,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "gbs_host.hpp"
@@ -270,33 +271,10 @@ gbs_status prepare_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, cons
     return GBS_OK;
 }
 
-gbs_status alloc_workspace(Workspace &w, uint32_t n_cap, uint64_t m_cap, cudaStream_t s) {
-    const size_t n = n_cap ? n_cap : 1;
-    GBS_CUDA(cudaMalloc(&w.dp, sizeof(unsigned long long) * n));
-    GBS_CUDA(cudaMalloc(&w.tag, sizeof(uint32_t) * n));
-    GBS_CUDA(cudaMalloc(&w.fst, sizeof(uint32_t) * n));
-    GBS_CUDA(cudaMalloc(&w.hst, sizeof(uint32_t) * n));
-    GBS_CUDA(cudaMalloc(&w.ring, sizeof(uint32_t) * n * kNB));
-    GBS_CUDA(cudaMalloc(&w.fq, sizeof(uint32_t) * n * 3));
-    GBS_CUDA(cudaMalloc(&w.pend, sizeof(uint32_t) * n * 2));
-    // a SCAN reads at most n entries and cuts each row into ceil(len/kDescEdges)
-    // descriptors, so it emits at most n + m/kDescEdges of them
-    const uint64_t cap = (uint64_t)n_cap + m_cap / kDescEdges + 64;
-    w.desc_cap = (uint32_t)std::min<uint64_t>(cap, 0xFFFFFFF0ull);
-    GBS_CUDA(cudaMalloc(&w.desc, sizeof(uint4) * (size_t)w.desc_cap));
-    GBS_CUDA(cudaMalloc(&w.hdesc, sizeof(uint4) * (size_t)w.desc_cap));
-    GBS_CUDA(cudaMalloc(&w.ctl, sizeof(Ctl)));
-    GBS_CUDA(cudaMemsetAsync(w.fst, 0, sizeof(uint32_t) * n, s));
-    GBS_CUDA(cudaMemsetAsync(w.hst, 0, sizeof(uint32_t) * n, s));
-    GBS_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), s));
-    w.n_cap = n_cap;
-    return GBS_OK;
-}
-
-void free_workspace(Workspace &w) {
-    cudaFree(w.dp); cudaFree(w.tag); cudaFree(w.fst); cudaFree(w.hst);
-    cudaFree(w.ring); cudaFree(w.fq); cudaFree(w.pend); cudaFree(w.desc); cudaFree(w.hdesc); cudaFree(w.ctl);
-    w = Workspace{};
+// a SCAN reads at most n entries and cuts each row into ceil(len/kDescEdges)
+// descriptors, so it emits at most n + m/kDescEdges of them
+uint32_t desc_capacity(uint32_t n_cap, uint64_t m_cap) {
+    return (uint32_t)std::min<uint64_t>((uint64_t)n_cap + m_cap / kDescEdges + 64, 0xFFFFFFF0ull);
 }
 
 int persistent_ctas_per_sm(gbs_weight_type wt, bool batch) {
@@ -328,14 +306,46 @@ gbs_status launch_mid(const uint32_t *row, const uint2 *adj, uint32_t n, uint32_
 
 gbs_status ensure_workspace(gbs_graph *g) {
     if (g->ws_ready) return GBS_OK;
+    // one allocation: a cudaMalloc of a few MB takes 35 us here, its cudaFree
+    // 35-140, and there were thirteen
     const size_t n = g->n ? g->n : 1;
-    gbs_status st = alloc_workspace(g->ws, g->n, g->m, g->stream);
-    if (st != GBS_OK) return st;
-    GBS_CUDA(cudaMalloc(&g->ws.mid, sizeof(uint32_t) * n));
-    g->ws.trace = nullptr;
-    g->ws.trace_cap = 0;
-    GBS_CUDA(cudaMalloc(&g->d_dist, dist_bytes(g->wtype) * n));
-    GBS_CUDA(cudaMalloc(&g->d_pred, sizeof(int32_t) * n));
+    Workspace w{};
+    w.desc_cap = desc_capacity(g->n, g->m);
+    w.n_cap = g->n;
+    size_t used = 0;
+    unsigned char *base = nullptr;
+    auto lay = [&](auto **p, size_t count) {
+        if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + used);
+        used += (sizeof(**p) * count + 255) & ~(size_t)255;
+    };
+    unsigned char *dist = nullptr;
+    int32_t *pred = nullptr;
+    auto lay_all = [&]() {
+        used = 0;
+        lay(&w.dp, n);
+        lay(&w.tag, n);
+        lay(&w.fst, n);
+        lay(&w.hst, n);
+        lay(&w.ring, n * kNB);
+        lay(&w.fq, n * 3);
+        lay(&w.pend, n * 2);
+        lay(&w.desc, w.desc_cap);
+        lay(&w.hdesc, w.desc_cap);
+        lay(&w.ctl, 1);
+        lay(&w.mid, n);
+        lay(&dist, dist_bytes(g->wtype) * n);
+        lay(&pred, n);
+    };
+    lay_all();
+    GBS_CUDA(cudaMalloc(&base, used));
+    lay_all();
+    g->ws_mem = base;
+    g->ws = w;
+    g->d_dist = reinterpret_cast<uint32_t *>(dist);
+    g->d_pred = pred;
+    GBS_CUDA(cudaMemsetAsync(w.fst, 0, sizeof(uint32_t) * n, g->stream));
+    GBS_CUDA(cudaMemsetAsync(w.hst, 0, sizeof(uint32_t) * n, g->stream));
+    GBS_CUDA(cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), g->stream));
     g->epoch = 1;
     g->hround = 1;
     const int per_sm = persistent_ctas_per_sm(g->wtype, false);
@@ -350,11 +360,8 @@ void free_graph(gbs_graph *g) {
     cudaFree(g->d_row);
     cudaFree(g->d_adj);
     cudaFree(g->d_w64);
-    cudaFree(g->ws.mid);
     cudaFree(g->ws.trace);
-    free_workspace(g->ws);
-    cudaFree(g->d_dist);
-    cudaFree(g->d_pred);
+    cudaFree(g->ws_mem);
     cudaFree(g->d_mlp);
     cudaFree(g->d_feat);
     cudaFreeHost(g->h_small);

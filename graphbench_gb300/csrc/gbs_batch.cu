@@ -133,8 +133,7 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 // m_cap edges; carve() lays it out in the same order.
 size_t workspace_bytes(uint32_t n_cap, uint64_t m_cap, uint32_t *desc_cap) {
     const size_t n = n_cap ? n_cap : 1;
-    const uint64_t cap = (uint64_t)n_cap + m_cap / kDescEdges + 64;
-    *desc_cap = (uint32_t)std::min<uint64_t>(cap, 0xFFFFFFF0ull);
+    *desc_cap = desc_capacity(n_cap, m_cap);
     size_t b = 0;
     b += align_up(8 * n);                 // dp
     b += 3 * align_up(4 * n);             // tag, fst, hst

@@ -45,6 +45,7 @@ struct gbs_graph {
     // workspace
     bool ws_ready = false;
     gbs::Workspace ws{};
+    void *ws_mem = nullptr;                 // the workspace, d_dist and d_pred
     uint32_t *d_dist = nullptr;
     int32_t *d_pred = nullptr;
     unsigned long long mid_light_key = 0;   // light bound the cached split index was built for
@@ -121,11 +122,9 @@ gbs_status prepare_csr(uint32_t n, uint64_t m, const uint64_t *row_offsets, cons
 gbs_status launch_mid(const uint32_t *row, const uint2 *adj, uint32_t n, uint32_t light_bits, uint32_t *mid,
                       int sms, cudaStream_t s);
 
-// Allocates the lists of a workspace for graphs of at most n_cap vertices
-// and m_cap edges (dp, tag, fst, hst, ring, fq, S, pend, desc, ctl; fst, hst
-// and ctl zeroed).  mid and trace are left to the caller.
-gbs_status alloc_workspace(Workspace &w, uint32_t n_cap, uint64_t m_cap, cudaStream_t s);
-void free_workspace(Workspace &w);
+// Descriptors one SCAN can emit on graphs of at most n_cap vertices and m_cap
+// edges: the capacity of a workspace's desc and hdesc.
+uint32_t desc_capacity(uint32_t n_cap, uint64_t m_cap);
 
 // Resident CTAs of the persistent kernels on one SM (0 if they cannot run).
 int persistent_ctas_per_sm(gbs_weight_type wt, bool batch);

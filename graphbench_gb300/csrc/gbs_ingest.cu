@@ -22,13 +22,19 @@
 // odd p (:293-298).  With dedup, a (from, to) pair seen earlier in the file is
 // dropped first, as remove_duplicate does.
 //
-// Device work: the text is cut into 512-byte chunks; each chunk counts and
-// then lists the "a" lines that start in it (one exclusive scan between), and
-// one thread per line parses its numbers.  The CSR is a stable radix sort of
-// the edges by row (CUB), so rows keep file order; the resident graph's rows
-// are then sorted by (weight, column) with two or three more stable passes.
+// Device work: the text is cut into 512-byte chunks; a warp counts and then
+// lists the "a" lines of a chunk, 16 bytes a lane (one exclusive scan between),
+// and one thread per line parses its numbers into a row, a column and a weight.
+// The CSR is a stable radix sort of the columns by row (CUB), so rows keep file
+// order; a file already in row order is not sorted.  The row offsets are
+// searched for in the sorted rows.  Duplicate removal sorts the pairs by the
+// bits their largest ids use.  Every call takes its buffers from one
+// allocation: a cudaMalloc of a few MB takes 35 us here, its cudaFree 35-140,
+// and a call has more than ten.  R-MAT of 65,536 vertices, 30 MB of text: copy,
+// lines and numbers 0.76 -> 0.27 ms (a thread per chunk read byte by byte),
+// build 0.68 -> 0.15, the call 1.9 -> 0.67; 3.1 M pairs with duplicates: 3.0 ->
+// 1.3.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include <chrono>
@@ -44,7 +50,7 @@
 namespace gbs {
 namespace {
 
-constexpr uint64_t kChunk = 512;     // bytes of text per counting thread
+constexpr uint64_t kChunk = 512;     // bytes of text per counting warp
 
 enum IngestErr : uint32_t {
     kIngOk = 0,
@@ -73,26 +79,51 @@ __device__ __forceinline__ bool a_line_at(const char *buf, unsigned long long le
     return i + 1 < len && buf[i] == 'a' && (buf[i + 1] == ' ' || buf[i + 1] == '\t');
 }
 
-__global__ void k_count_lines(const char *__restrict__ buf, unsigned long long len, unsigned long long chunks,
-                              unsigned long long *__restrict__ cnt) {
-    for (unsigned long long c = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; c < chunks;
-         c += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long b = c * kChunk, e = min(len, b + kChunk);
-        unsigned long long k = 0;
-        for (unsigned long long i = b; i < e; ++i) k += a_line_at(buf, len, i) ? 1ull : 0ull;
-        cnt[c] = k;
-    }
-}
-
-__global__ void k_list_lines(const char *__restrict__ buf, unsigned long long len, unsigned long long chunks,
-                             const unsigned long long *__restrict__ base, unsigned long long *__restrict__ pos,
-                             unsigned long long cap) {
-    for (unsigned long long c = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; c < chunks;
-         c += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long b = c * kChunk, e = min(len, b + kChunk);
-        unsigned long long k = base[c];
-        for (unsigned long long i = b; i < e && k < cap; ++i)
-            if (a_line_at(buf, len, i)) pos[k++] = i;
+// The "a" records whose preceding newline (or the start of the file) lies in a
+// chunk: counted, or listed from base[chunk] on.  A warp takes a chunk, a lane
+// 16 bytes of it (buf is padded to whole 16-byte groups).
+template <bool List>
+__global__ void __launch_bounds__(256) k_lines(const char *__restrict__ buf, unsigned long long len,
+                                               unsigned long long chunks, unsigned long long *__restrict__ cnt,
+                                               const unsigned long long *__restrict__ base,
+                                               unsigned long long *__restrict__ pos, unsigned long long cap) {
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
+    const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    for (unsigned long long c = warp; c < chunks; c += warps) {
+        const unsigned long long at = c * kChunk + 16ull * lane;
+        uint32_t starts = 0;   // bit j: a record starts at at + j + 1; bit 16: at 0
+        if (at < len) {
+            const uint4 x = *reinterpret_cast<const uint4 *>(buf + at);
+            const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (((w[j >> 2] >> (8 * (j & 3))) & 0xFFu) == '\n' && at + j < len) starts |= 1u << j;
+            for (uint32_t b = starts; b; b &= b - 1u) {
+                const int j = __ffs((int)b) - 1;
+                if (!a_line_at(buf, len, at + j + 1ull)) starts &= ~(1u << j);
+            }
+            if (at == 0ull && a_line_at(buf, len, 0ull)) starts |= 1u << 16;
+        }
+        const uint32_t n = (uint32_t)__popc(starts);
+        if (!List) {
+            const uint32_t total = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0) cnt[c] = total;
+        } else {
+            uint32_t incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)lane >= o) incl += y;
+            }
+            unsigned long long k = base[c] + incl - n;
+            if (starts & (1u << 16)) {   // the start of the file comes before its first newline
+                if (k < cap) pos[k] = 0ull;
+                ++k;
+            }
+            for (uint32_t b = starts & 0xFFFFu; b; b &= b - 1u, ++k)
+                if (k < cap) pos[k] = at + (unsigned long long)__ffs((int)b);
+        }
     }
 }
 
@@ -112,11 +143,27 @@ __device__ __forceinline__ bool read_int(const char *buf, unsigned long long len
     return true;
 }
 
-// One thread per "a" record: v_id and v_to (the weight token is checked and
-// ignored, as the reference ignores it).
+// Row and column of an edge, checked against [0, v_num).
+__device__ __forceinline__ void put_edge(long long r, long long c, long long v_num, unsigned long long k,
+                                         uint32_t *__restrict__ row, uint32_t *__restrict__ col, DevErr *err) {
+    if (r < 0 || r >= v_num || c < 0 || c >= v_num) {
+        set_err(err, kIngRange, k);
+        r = c = 0;
+    }
+    row[k] = (uint32_t)r;
+    col[k] = (uint32_t)c;
+}
+
+// One thread per "a" record, at most cap of them: row, column, and the weight
+// of CSR position k, the k-th line's v_to / v_num (the weight token is checked
+// and ignored, as the reference ignores it).  err[0]: a malformed line, err[1]:
+// an edge out of range.
 __global__ void k_parse_lines(const char *__restrict__ buf, unsigned long long len,
-                              const unsigned long long *__restrict__ pos, unsigned long long count,
-                              long long *__restrict__ x, long long *__restrict__ y, DevErr *err) {
+                              const unsigned long long *__restrict__ pos, const unsigned long long *__restrict__ lines,
+                              unsigned long long cap, long long row_shift, bool by_to, long long v_num,
+                              uint32_t *__restrict__ row, uint32_t *__restrict__ col, double *__restrict__ wout,
+                              DevErr *err) {
+    const unsigned long long count = min(*lines, cap);
     for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < count;
          k += (unsigned long long)gridDim.x * blockDim.x) {
         unsigned long long i = pos[k];
@@ -125,65 +172,83 @@ __global__ void k_parse_lines(const char *__restrict__ buf, unsigned long long l
         long long a = 0, b = 0, w = 0;
         if (!read_int(buf, len, i, a) || !read_int(buf, len, i, b) || !read_int(buf, len, i, w)) {
             set_err(err, kIngSyntax, k);
+            row[k] = col[k] = 0u;
             continue;
         }
-        x[k] = a;
-        y[k] = b;
+        put_edge((by_to ? b : a) - row_shift, (by_to ? a : b) - 1, v_num, k, row, col, err + 1);
+        wout[k] = (double)b / (double)v_num;
     }
 }
 
-// Row and column of every edge (file order), checked against [0, v_num).
-__global__ void k_rows(const long long *__restrict__ x, const long long *__restrict__ y, unsigned long long m,
-                       long long row_shift, long long col_shift, bool by_y, long long v_num,
-                       uint32_t *__restrict__ row, uint32_t *__restrict__ col, uint32_t *__restrict__ idx,
-                       DevErr *err) {
+// Binary pairs: all of them, or (keep given) pair k as edge at[k] where keep[k] is set.
+__global__ void k_pair_rows(const longlong2 *__restrict__ pairs, unsigned long long m, const uint32_t *__restrict__ keep,
+                            const uint32_t *__restrict__ at, long long row_shift, long long col_shift, bool by_to,
+                            long long v_num, uint32_t *__restrict__ row, uint32_t *__restrict__ col, DevErr *err) {
     for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
          k += (unsigned long long)gridDim.x * blockDim.x) {
-        const long long r = (by_y ? y[k] : x[k]) - row_shift;
-        const long long c = (by_y ? x[k] : y[k]) - col_shift;
-        if (r < 0 || r >= v_num || c < 0 || c >= v_num) {
-            set_err(err, kIngRange, k);
-            row[k] = 0;
-            col[k] = 0;
-        } else {
-            row[k] = (uint32_t)r;
-            col[k] = (uint32_t)c;
-        }
-        idx[k] = (uint32_t)k;
+        if (keep && !keep[k]) continue;
+        const longlong2 p = pairs[k];
+        put_edge((by_to ? p.y : p.x) - row_shift, (by_to ? p.x : p.y) - col_shift, v_num, keep ? at[k] : k, row, col, err);
     }
 }
 
-__global__ void k_degrees(const uint32_t *__restrict__ row, unsigned long long m, unsigned long long *__restrict__ deg) {
-    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
+// Whether the rows are not in ascending order.
+__global__ void k_row_order(const uint32_t *__restrict__ row, unsigned long long m, uint32_t *unsorted) {
+    bool bad = false;
+    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x + 1ull; k < m;
          k += (unsigned long long)gridDim.x * blockDim.x)
-        atomicAdd(deg + row[k], 1ull);
+        bad |= row[k] < row[k - 1ull];
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31u) == 0) *unsorted = 1u;
 }
 
-// CSR position p: the column of the p-th edge in (row, file order); the
-// weight as the reference stores it (text: the p-th line's v_to / v_num;
-// binary: 0.1 / 0.2 by the parity of p).
-__global__ void k_place(const uint32_t *__restrict__ sorted_idx, const uint32_t *__restrict__ col,
-                        const long long *__restrict__ raw_to, unsigned long long m, bool text, double v_num,
-                        uint32_t *__restrict__ out_col, double *__restrict__ out_w) {
-    for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
-         p += (unsigned long long)gridDim.x * blockDim.x) {
-        out_col[p] = col[sorted_idx[p]];
-        out_w[p] = text ? (double)raw_to[p] / v_num : ((p & 1ull) ? 0.2 : 0.1);
+// out[v] = the first position of row v or a later one.
+__global__ void k_row_starts(const uint32_t *__restrict__ row, unsigned long long m, uint32_t n,
+                             unsigned long long *__restrict__ out) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x) {
+        unsigned long long lo = 0ull, hi = m;
+        while (lo < hi) {
+            const unsigned long long mid = lo + (hi - lo) / 2ull;
+            if (row[mid] < v) lo = mid + 1ull;
+            else hi = mid;
+        }
+        out[v] = lo;
     }
 }
 
-// Duplicate removal: key = (from << 32) | to of the raw pair.
-__global__ void k_pair_keys(const long long *__restrict__ x, const long long *__restrict__ y, unsigned long long m,
-                            unsigned long long *__restrict__ key, uint32_t *__restrict__ idx, DevErr *err) {
+// Binary files: the weight of CSR position p is 0.1 for even p, 0.2 for odd p.
+__global__ void k_parity_weights(unsigned long long m, double *__restrict__ out) {
+    for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
+         p += (unsigned long long)gridDim.x * blockDim.x)
+        out[p] = (p & 1ull) ? 0.2 : 0.1;
+}
+
+// Duplicate removal: the largest ids of the raw pairs, which must be in
+// [0, 2^32); then key = from << to_bits | to.
+__global__ void k_pair_max(const longlong2 *__restrict__ pairs, unsigned long long m, uint32_t *mx, DevErr *err) {
+    uint32_t a = 0, b = 0;
     for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
          k += (unsigned long long)gridDim.x * blockDim.x) {
-        const long long a = x[k], b = y[k];
-        if (a < 0 || b < 0 || a > 0xFFFFFFFFll || b > 0xFFFFFFFFll) {
+        const longlong2 p = pairs[k];
+        if (p.x < 0 || p.y < 0 || p.x > 0xFFFFFFFFll || p.y > 0xFFFFFFFFll) {
             set_err(err, kIngDupRange, k);
-            key[k] = 0;
         } else {
-            key[k] = ((unsigned long long)a << 32) | (unsigned long long)b;
+            a = max(a, (uint32_t)p.x);
+            b = max(b, (uint32_t)p.y);
         }
+    }
+    a = __reduce_max_sync(0xffffffffu, a);
+    b = __reduce_max_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31u) == 0) {
+        atomicMax(mx, a);
+        atomicMax(mx + 1, b);
+    }
+}
+__global__ void k_pair_keys(const longlong2 *__restrict__ pairs, unsigned long long m, int to_bits,
+                            unsigned long long *__restrict__ key, uint32_t *__restrict__ idx) {
+    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
+         k += (unsigned long long)gridDim.x * blockDim.x) {
+        const longlong2 p = pairs[k];
+        key[k] = ((unsigned long long)p.x << to_bits) | (unsigned long long)p.y;
         idx[k] = (uint32_t)k;
     }
 }
@@ -195,32 +260,6 @@ __global__ void k_first_of_run(const unsigned long long *__restrict__ key, const
     for (unsigned long long p = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; p < m;
          p += (unsigned long long)gridDim.x * blockDim.x)
         keep[idx[p]] = (p == 0 || key[p] != key[p - 1]) ? 1u : 0u;
-}
-
-__global__ void k_compact(const long long *__restrict__ x, const long long *__restrict__ y,
-                          const uint32_t *__restrict__ keep, const unsigned long long *__restrict__ at,
-                          unsigned long long m, long long *__restrict__ ox, long long *__restrict__ oy) {
-    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
-         k += (unsigned long long)gridDim.x * blockDim.x)
-        if (keep[k]) {
-            ox[at[k]] = x[k];
-            oy[at[k]] = y[k];
-        }
-}
-
-__global__ void k_widen(const uint32_t *__restrict__ in, unsigned long long m, unsigned long long *__restrict__ out) {
-    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k <= m;
-         k += (unsigned long long)gridDim.x * blockDim.x)
-        out[k] = k < m ? in[k] : 0ull;
-}
-
-__global__ void k_split(const long long *__restrict__ pairs, unsigned long long m, long long *__restrict__ x,
-                        long long *__restrict__ y) {
-    for (unsigned long long k = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; k < m;
-         k += (unsigned long long)gridDim.x * blockDim.x) {
-        x[k] = pairs[2 * k];
-        y[k] = pairs[2 * k + 1];
-    }
 }
 
 // ------------------------------------------------- resident graph build
@@ -367,25 +406,45 @@ __global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, 
 }
 
 // ----------------------------------------------------------------- host
-// Device buffers of one ingest call, released on every exit path.
+// Device buffers of one call, released on every exit path: taken from one
+// block where it was reserved and holds them (a stack: reset gives back what was
+// taken since the mark, for later work on the same stream), allocated one by one
+// otherwise.  Calls beyond kMaxBlock do not reserve: freeing each buffer when
+// it is done keeps their peak lower.
+constexpr size_t kMaxBlock = 8ull << 30;
 struct Bufs {
-    std::vector<void *> p;
+    std::vector<void *> own;
+    char *block = nullptr;
+    size_t cap = 0, used = 0;
+    void reserve(size_t bytes) {
+        if (block || bytes > kMaxBlock) return;
+        if (cudaMalloc(reinterpret_cast<void **>(&block), bytes) == cudaSuccess) cap = bytes;
+        else cudaGetLastError();
+    }
     template <typename T> cudaError_t get(T **out, size_t count) {
+        const size_t bytes = (sizeof(T) * (count ? count : 1) + 255) & ~(size_t)255;
+        if (used + bytes <= cap) {
+            *out = reinterpret_cast<T *>(block + used);
+            used += bytes;
+            return cudaSuccess;
+        }
         void *q = nullptr;
-        const cudaError_t e = cudaMalloc(&q, sizeof(T) * (count ? count : 1));
-        if (e == cudaSuccess) p.push_back(q);
+        const cudaError_t e = cudaMalloc(&q, bytes);
+        if (e == cudaSuccess) own.push_back(q);
         *out = static_cast<T *>(q);
         return e;
     }
-    void release(void *q) {
-        for (auto &x : p)
-            if (x == q) {
-                cudaFree(x);
-                x = nullptr;
-            }
+    struct Mark {
+        size_t used, own;
+    };
+    Mark mark() const { return {used, own.size()}; }
+    void reset(Mark m) {
+        used = m.used;
+        for (; own.size() > m.own; own.pop_back()) cudaFree(own.back());
     }
     ~Bufs() {
-        for (void *q : p) cudaFree(q);
+        reset({0, 0});
+        cudaFree(block);
     }
 };
 
@@ -418,66 +477,58 @@ gbs_status check_err(const DevErr &e, const char *what) {
 template <typename K>
 gbs_status sort_pairs(const K *kin, K *kout, const uint32_t *vin, uint32_t *vout, unsigned long long m,
                       cudaStream_t s, Bufs &bufs, int end_bit = (int)sizeof(K) * 8) {
+    const Bufs::Mark at = bufs.mark();
     size_t tmp = 0;
     ING_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, kin, kout, vin, vout, (int64_t)m, 0, end_bit, s));
     void *t = nullptr;
     ING_CUDA(bufs.get(reinterpret_cast<char **>(&t), tmp));
     ING_CUDA(cub::DeviceRadixSort::SortPairs(t, tmp, kin, kout, vin, vout, (int64_t)m, 0, end_bit, s));
-    bufs.release(t);
+    bufs.reset(at);
     return GBS_OK;
 }
 
-gbs_status excl_sum(const unsigned long long *in, unsigned long long *out, unsigned long long count, cudaStream_t s,
-                    Bufs &bufs) {
+template <typename T>
+gbs_status excl_sum(const T *in, T *out, unsigned long long count, cudaStream_t s, Bufs &bufs) {
+    const Bufs::Mark at = bufs.mark();
     size_t tmp = 0;
     ING_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, in, out, (int64_t)count, s));
     void *t = nullptr;
     ING_CUDA(bufs.get(reinterpret_cast<char **>(&t), tmp));
     ING_CUDA(cub::DeviceScan::ExclusiveSum(t, tmp, in, out, (int64_t)count, s));
-    bufs.release(t);
+    bufs.reset(at);
     return GBS_OK;
 }
 
-// Edges (x, y) in file order -> CSR in the reference's layout.
-gbs_status build_csr(const long long *dx, const long long *dy, unsigned long long m, long long v_num, long long row_shift,
-                     long long col_shift, bool by_y, bool text, cudaStream_t s, int sms, Bufs &bufs,
-                     gbs_device_csr *out) {
-    DevErr *d_err = nullptr;
-    ING_CUDA(bufs.get(&d_err, 1));
-    ING_CUDA(cudaMemsetAsync(d_err, 0, sizeof(DevErr), s));
-    uint32_t *row = nullptr, *col = nullptr, *idx = nullptr, *row_s = nullptr, *idx_s = nullptr;
-    ING_CUDA(bufs.get(&row, m));
-    ING_CUDA(bufs.get(&col, m));
-    ING_CUDA(bufs.get(&idx, m));
-    const int gb = grid_for(m, sms);
-    k_rows<<<gb, 256, 0, s>>>(dx, dy, m, row_shift, col_shift, by_y, v_num, row, col, idx, d_err);
+int bits_of(unsigned long long most) {   // bits of the values 0 .. most, at least 1
+    int b = 1;
+    while (b < 64 && (most >> b)) ++b;
+    return b;
+}
+
+// Edges (row, col) in file order -> the CSR's offsets and columns, rows in file
+// order.  `unsorted`: a device word the call may use.
+gbs_status build_csr(const uint32_t *row, const uint32_t *col, unsigned long long m, uint32_t n, uint32_t *unsorted,
+                     cudaStream_t s, int sms, Bufs &bufs, gbs_device_csr *out) {
+    uint32_t hu = 0;
+    ING_CUDA(cudaMemsetAsync(unsorted, 0, sizeof(uint32_t), s));
+    k_row_order<<<grid_for(m, sms), 256, 0, s>>>(row, m, unsorted);
     ING_CUDA(cudaGetLastError());
-    DevErr he{};
-    ING_CUDA(cudaMemcpyAsync(&he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
-    ING_CUDA(cudaStreamSynchronize(s));
-    gbs_status st = check_err(he, text ? "text graph" : "binary graph");
-    if (st != GBS_OK) return st;
-    unsigned long long *deg = nullptr;
-    ING_CUDA(bufs.get(&deg, (size_t)v_num + 1));
-    ING_CUDA(cudaMemsetAsync(deg, 0, sizeof(unsigned long long) * ((size_t)v_num + 1), s));
-    k_degrees<<<gb, 256, 0, s>>>(row, m, deg);
-    ING_CUDA(cudaGetLastError());
-    ING_CUDA(cudaMalloc(&out->d_row, sizeof(unsigned long long) * ((size_t)v_num + 1)));
-    st = excl_sum(deg, out->d_row, (unsigned long long)v_num + 1, s, bufs);
-    if (st != GBS_OK) return st;
-    ING_CUDA(bufs.get(&row_s, m));
-    ING_CUDA(bufs.get(&idx_s, m));
-    int bits = 1;
-    while (bits < 32 && (1ll << bits) < v_num) ++bits;
-    st = sort_pairs<uint32_t>(row, row_s, idx, idx_s, m, s, bufs, bits);
-    if (st != GBS_OK) return st;
+    ING_CUDA(cudaMemcpyAsync(&hu, unsorted, sizeof(hu), cudaMemcpyDeviceToHost, s));
+    ING_CUDA(cudaMalloc(&out->d_row, sizeof(unsigned long long) * ((size_t)n + 1)));
     ING_CUDA(cudaMalloc(&out->d_col, sizeof(uint32_t) * (m ? m : 1)));
-    ING_CUDA(cudaMalloc(&out->d_w, sizeof(double) * (m ? m : 1)));
-    // text weights come from the raw v_to of each line, in file order
-    k_place<<<gb, 256, 0, s>>>(idx_s, col, dy, m, text, (double)v_num, out->d_col, out->d_w);
-    ING_CUDA(cudaGetLastError());
     ING_CUDA(cudaStreamSynchronize(s));
-    out->n = (uint32_t)v_num;
+    if (hu) {
+        uint32_t *row_s = nullptr;
+        ING_CUDA(bufs.get(&row_s, m));
+        const gbs_status st = sort_pairs<uint32_t>(row, row_s, col, out->d_col, m, s, bufs, bits_of(n - 1u));
+        if (st != GBS_OK) return st;
+        row = row_s;
+    } else {
+        ING_CUDA(cudaMemcpyAsync(out->d_col, col, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, s));
+    }
+    k_row_starts<<<grid_for((unsigned long long)n + 1, sms), 256, 0, s>>>(row, m, n, out->d_row);
+    ING_CUDA(cudaGetLastError());
+    out->n = n;
     out->m = m;
     return GBS_OK;
 }
@@ -573,47 +624,50 @@ gbs_status ingest_text(const char *bytes, size_t len, int direction, gbs_device_
             for (int i = 0; i < 3; ++i) cudaEventDestroy(e[i]);
         }
     } ef{ev};
-    char *dbuf = nullptr;
-    ING_CUDA(bufs.get(&dbuf, len + 1));
-    ING_CUDA(cudaEventRecord(ev[0], s));
-    ING_CUDA(cudaMemcpyAsync(dbuf, bytes, len, cudaMemcpyHostToDevice, s));
+    // the reference stops after e_num records, and none is shorter than "a 1 1 1"
+    const unsigned long long cap = std::min<unsigned long long>((unsigned long long)hdr[1], len / 7 + 1);
     const unsigned long long chunks = (len + kChunk - 1) / kChunk;
-    unsigned long long *cnt = nullptr, *base = nullptr;
+    bufs.reserve(len + 16 * chunks + 36 * cap + (4u << 20));
+    char *dbuf = nullptr;
+    unsigned long long *cnt = nullptr, *base = nullptr, *pos = nullptr;
+    uint32_t *row = nullptr, *col = nullptr, *word = nullptr;
+    DevErr *d_err = nullptr;
+    ING_CUDA(bufs.get(&word, 1));
+    ING_CUDA(bufs.get(&d_err, 2));
+    ING_CUDA(bufs.get(&row, cap));
+    ING_CUDA(bufs.get(&col, cap));
+    ING_CUDA(cudaMalloc(&out->d_w, sizeof(double) * (cap ? cap : 1)));
+    const Bufs::Mark parse = bufs.mark();
+    ING_CUDA(bufs.get(&dbuf, len + 16));
     ING_CUDA(bufs.get(&cnt, chunks + 1));
     ING_CUDA(bufs.get(&base, chunks + 1));
-    ING_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * (chunks + 1), s));
-    k_count_lines<<<grid_for(chunks, sms), 256, 0, s>>>(dbuf, len, chunks, cnt);
+    ING_CUDA(bufs.get(&pos, cap));
+    ING_CUDA(cudaEventRecord(ev[0], s));
+    ING_CUDA(cudaMemcpyAsync(dbuf, bytes, len, cudaMemcpyHostToDevice, s));
+    ING_CUDA(cudaMemsetAsync(cnt + chunks, 0, sizeof(unsigned long long), s));
+    ING_CUDA(cudaMemsetAsync(d_err, 0, 2 * sizeof(DevErr), s));
+    const int gc = grid_for(chunks * 32, sms);
+    k_lines<false><<<gc, 256, 0, s>>>(dbuf, len, chunks, cnt, nullptr, nullptr, 0);
     ING_CUDA(cudaGetLastError());
     st = excl_sum(cnt, base, chunks + 1, s, bufs);
     if (st != GBS_OK) return st;
+    // SEND: row = v_id - offset, col = v_to - 1; RECV: row = v_to - offset, col = v_id - 1
+    const bool send = direction != GBS_DIR_RECV;
+    k_lines<true><<<gc, 256, 0, s>>>(dbuf, len, chunks, nullptr, base, pos, cap);
+    k_parse_lines<<<grid_for(cap, sms), 256, 0, s>>>(dbuf, len, pos, base + chunks, cap, hdr[2], !send, hdr[0], row, col,
+                                                     out->d_w, d_err);
+    ING_CUDA(cudaGetLastError());
     unsigned long long lines = 0;
+    DevErr he[2] = {};
     ING_CUDA(cudaMemcpyAsync(&lines, base + chunks, sizeof(lines), cudaMemcpyDeviceToHost, s));
-    ING_CUDA(cudaStreamSynchronize(s));
-    // the reference stops after e_num records
-    const unsigned long long m = std::min<unsigned long long>(lines, (unsigned long long)hdr[1]);
-    unsigned long long *pos = nullptr;
-    ING_CUDA(bufs.get(&pos, m));
-    k_list_lines<<<grid_for(chunks, sms), 256, 0, s>>>(dbuf, len, chunks, base, pos, m);
-    ING_CUDA(cudaGetLastError());
-    long long *dx = nullptr, *dy = nullptr;
-    ING_CUDA(bufs.get(&dx, m));
-    ING_CUDA(bufs.get(&dy, m));
-    DevErr *d_err = nullptr;
-    ING_CUDA(bufs.get(&d_err, 1));
-    ING_CUDA(cudaMemsetAsync(d_err, 0, sizeof(DevErr), s));
-    k_parse_lines<<<grid_for(m, sms), 256, 0, s>>>(dbuf, len, pos, m, dx, dy, d_err);
-    ING_CUDA(cudaGetLastError());
-    DevErr he{};
-    ING_CUDA(cudaMemcpyAsync(&he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
+    ING_CUDA(cudaMemcpyAsync(he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
     ING_CUDA(cudaEventRecord(ev[1], s));
     ING_CUDA(cudaStreamSynchronize(s));
-    st = check_err(he, "text graph");
-    if (st != GBS_OK) return st;
-    bufs.release(dbuf);
-    bufs.release(pos);
-    const bool send = direction != GBS_DIR_RECV;
-    // SEND: row = v_id - offset, col = v_to - 1; RECV: row = v_to - offset, col = v_id - 1
-    st = build_csr(dx, dy, m, hdr[0], hdr[2], 1, !send, true, s, sms, bufs, out);
+    for (const DevErr &e : he)
+        if ((st = check_err(e, "text graph")) != GBS_OK) return st;
+    const unsigned long long m = std::min(lines, cap);
+    bufs.reset(parse);
+    st = build_csr(row, col, m, (uint32_t)hdr[0], word, s, sms, bufs, out);
     if (st != GBS_OK) return st;
     ING_CUDA(cudaEventRecord(ev[2], s));
     ING_CUDA(cudaEventSynchronize(ev[2]));
@@ -661,70 +715,70 @@ gbs_status ingest_bin(const char *bytes, size_t len, int direction, long long ta
             for (int i = 0; i < 3; ++i) cudaEventDestroy(e[i]);
         }
     } ef{ev};
-    // pairs are interleaved (from, to): copy both into one array, then split
-    long long *pairs = nullptr, *dx = nullptr, *dy = nullptr;
-    ING_CUDA(bufs.get(&pairs, 2 * m0));
-    ING_CUDA(bufs.get(&dx, m0));
-    ING_CUDA(bufs.get(&dy, m0));
+    bufs.reserve((dedup ? 70 : 38) * m0 + (16u << 20));
+    longlong2 *pairs = nullptr;
+    uint32_t *row = nullptr, *col = nullptr, *word = nullptr, *keep = nullptr, *at = nullptr;
+    DevErr *d_err = nullptr, he{};
+    ING_CUDA(bufs.get(&word, 2));
+    ING_CUDA(bufs.get(&d_err, 1));
+    ING_CUDA(bufs.get(&row, m0));
+    ING_CUDA(bufs.get(&col, m0));
+    const Bufs::Mark raw = bufs.mark();
+    ING_CUDA(bufs.get(&pairs, m0));
     ING_CUDA(cudaEventRecord(ev[0], s));
     ING_CUDA(cudaMemcpyAsync(pairs, bytes + 32, 16 * m0, cudaMemcpyHostToDevice, s));
-    k_split<<<grid_for(m0, sms), 256, 0, s>>>(pairs, m0, dx, dy);
-    ING_CUDA(cudaGetLastError());
-    ING_CUDA(cudaStreamSynchronize(s));
-    bufs.release(pairs);
-    unsigned long long m = m0, dups = 0;
+    ING_CUDA(cudaMemsetAsync(d_err, 0, sizeof(DevErr), s));
+    const int gb = grid_for(m0, sms);
+    unsigned long long m = m0;
     if (dedup && m0) {
-        unsigned long long *key = nullptr, *key_s = nullptr, *at = nullptr;
-        uint32_t *idx = nullptr, *idx_s = nullptr, *keep = nullptr;
-        DevErr *d_err = nullptr;
-        ING_CUDA(bufs.get(&d_err, 1));
-        ING_CUDA(cudaMemsetAsync(d_err, 0, sizeof(DevErr), s));
+        uint32_t mx[2] = {0, 0}, kept = 0;
+        ING_CUDA(cudaMemsetAsync(word, 0, 2 * sizeof(uint32_t), s));
+        k_pair_max<<<gb, 256, 0, s>>>(pairs, m0, word, d_err);
+        ING_CUDA(cudaGetLastError());
+        ING_CUDA(cudaMemcpyAsync(&he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
+        ING_CUDA(cudaMemcpyAsync(mx, word, sizeof(mx), cudaMemcpyDeviceToHost, s));
+        ING_CUDA(cudaStreamSynchronize(s));
+        st = check_err(he, "binary graph");
+        if (st != GBS_OK) return st;
+        ING_CUDA(bufs.get(&keep, m0 + 1));   // one more slot for the total
+        ING_CUDA(bufs.get(&at, m0 + 1));
+        const Bufs::Mark keys = bufs.mark();
+        unsigned long long *key = nullptr, *key_s = nullptr;
+        uint32_t *idx = nullptr, *idx_s = nullptr;
         ING_CUDA(bufs.get(&key, m0));
         ING_CUDA(bufs.get(&key_s, m0));
         ING_CUDA(bufs.get(&idx, m0));
         ING_CUDA(bufs.get(&idx_s, m0));
-        const int gb = grid_for(m0, sms);
-        k_pair_keys<<<gb, 256, 0, s>>>(dx, dy, m0, key, idx, d_err);
+        const int to_bits = bits_of(mx[1]);
+        k_pair_keys<<<gb, 256, 0, s>>>(pairs, m0, to_bits, key, idx);
         ING_CUDA(cudaGetLastError());
-        DevErr he{};
-        ING_CUDA(cudaMemcpyAsync(&he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
-        ING_CUDA(cudaStreamSynchronize(s));
-        st = check_err(he, "binary graph");
+        st = sort_pairs<unsigned long long>(key, key_s, idx, idx_s, m0, s, bufs, bits_of(mx[0]) + to_bits);
         if (st != GBS_OK) return st;
-        st = sort_pairs<unsigned long long>(key, key_s, idx, idx_s, m0, s, bufs);
-        if (st != GBS_OK) return st;
-        ING_CUDA(bufs.get(&keep, m0));
         k_first_of_run<<<gb, 256, 0, s>>>(key_s, idx_s, m0, keep);
         ING_CUDA(cudaGetLastError());
-        bufs.release(key);
-        bufs.release(key_s);
-        bufs.release(idx);
-        bufs.release(idx_s);
-        // keep flags widened to 64-bit counts, one more slot for the total
-        unsigned long long *keep64 = nullptr;
-        ING_CUDA(bufs.get(&keep64, m0 + 1));
-        k_widen<<<gb, 256, 0, s>>>(keep, m0, keep64);
-        ING_CUDA(cudaGetLastError());
-        ING_CUDA(bufs.get(&at, m0 + 1));
-        st = excl_sum(keep64, at, m0 + 1, s, bufs);
+        bufs.reset(keys);
+        ING_CUDA(cudaMemsetAsync(keep + m0, 0, sizeof(uint32_t), s));
+        st = excl_sum(keep, at, m0 + 1, s, bufs);
         if (st != GBS_OK) return st;
-        unsigned long long kept = 0;
         ING_CUDA(cudaMemcpyAsync(&kept, at + m0, sizeof(kept), cudaMemcpyDeviceToHost, s));
-        long long *ox = nullptr, *oy = nullptr;
-        ING_CUDA(bufs.get(&ox, m0));
-        ING_CUDA(bufs.get(&oy, m0));
-        k_compact<<<gb, 256, 0, s>>>(dx, dy, keep, at, m0, ox, oy);
-        ING_CUDA(cudaGetLastError());
         ING_CUDA(cudaStreamSynchronize(s));
-        dx = ox;
-        dy = oy;
         m = kept;
-        dups = m0 - kept;
     }
+    const unsigned long long dups = m0 - m;
     ING_CUDA(cudaEventRecord(ev[1], s));
-    const bool send = direction != GBS_DIR_RECV;
     // SEND: row = from - offset, col = to - target_offset; RECV: row = to - offset, col = from - target_offset
-    st = build_csr(dx, dy, m, hdr[0], hdr[2], target_offset, !send, false, s, sms, bufs, out);
+    const bool send = direction != GBS_DIR_RECV;
+    k_pair_rows<<<gb, 256, 0, s>>>(pairs, m0, keep, at, hdr[2], target_offset, !send, hdr[0], row, col, d_err);
+    ING_CUDA(cudaGetLastError());
+    ING_CUDA(cudaMemcpyAsync(&he, d_err, sizeof(he), cudaMemcpyDeviceToHost, s));
+    ING_CUDA(cudaStreamSynchronize(s));
+    st = check_err(he, "binary graph");
+    if (st != GBS_OK) return st;
+    bufs.reset(raw);
+    ING_CUDA(cudaMalloc(&out->d_w, sizeof(double) * (m ? m : 1)));
+    k_parity_weights<<<grid_for(m, sms), 256, 0, s>>>(m, out->d_w);
+    ING_CUDA(cudaGetLastError());
+    st = build_csr(row, col, m, (uint32_t)hdr[0], word, s, sms, bufs, out);
     if (st != GBS_OK) return st;
     ING_CUDA(cudaEventRecord(ev[2], s));
     ING_CUDA(cudaEventSynchronize(ev[2]));
@@ -757,12 +811,15 @@ __global__ void k_iota(uint32_t *__restrict__ id, unsigned long long m) {
 // messages); else from a device CSR.  gbs_graph_create, checked and sorted by 16
 // host cores -> here, ms: R-MAT 16 6.5 -> 1.1 (float64 10.8 -> 1.7), 20 116 ->
 // 5.6, 22 475 -> 20.
+size_t build_bytes(unsigned long long m, bool f64) { return (f64 ? 60 : 36) * m + (8u << 20); }
+
 template <int WT, typename Src>
 gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long long *row, const uint32_t *col, const Src *w,
                        bool host, int sms, cudaStream_t s, Bufs &bufs, gbs_graph **out) {
     constexpr gbs_weight_type wtype = WT == 2 ? GBS_WEIGHT_F64 : WT == 1 ? GBS_WEIGHT_F32 : GBS_WEIGHT_U32;
     constexpr bool f64 = WT == 2;
     const int gb = grid_for(m, sms);
+    bufs.reserve(build_bytes(m, f64));
     EdgeStats *st = nullptr, hs{};
     unsigned long long *key = nullptr, *key_s = nullptr;
     uint32_t *row_of = nullptr, *row32 = nullptr;
@@ -807,7 +864,7 @@ gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long lon
     uint32_t *id0 = nullptr, *id1 = nullptr, *col_s = nullptr;
     const uint32_t *cols = col;   // the columns in the order of the keys
     gbs_status r;
-    ING_CUDA(bufs.get(&col_s, m));
+    if (!f64 || hs.unsorted) ING_CUDA(bufs.get(&col_s, m));
     if (f64 || hs.unsorted) {
         ING_CUDA(bufs.get(&id0, m));
         ING_CUDA(bufs.get(&id1, m));
@@ -895,6 +952,7 @@ gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const ui
     unsigned long long *d_row = nullptr;
     uint32_t *d_col = nullptr;
     char *d_w = nullptr;
+    bufs.reserve(8ull * n + (4 + wb) * m + build_bytes(m, wtype == GBS_WEIGHT_F64));
     ING_CUDA(bufs.get(&d_row, (size_t)n + 1));
     ING_CUDA(bufs.get(&d_col, m));
     ING_CUDA(bufs.get(&d_w, wb * m));
