@@ -93,24 +93,38 @@ __global__ void k_unpack64(const unsigned long long *__restrict__ dp, uint32_t n
 }
 
 // float64 predecessors: the smallest u with an edge (u, v) and dist[u] + w ==
-// dist[v] in double (the same rounded add as the relaxation).  One warp per
-// row; every reached vertex other than the source has such an edge.
-__global__ void k_pred64(const uint32_t *__restrict__ row, const uint2 *__restrict__ adj,
-                         const unsigned long long *__restrict__ w64, const unsigned long long *__restrict__ dp,
-                         uint32_t n, uint32_t src, int32_t *__restrict__ pred) {
+// dist[v] in double (the same rounded add as the relaxation); every reached
+// vertex other than the source has such an edge.  A warp takes kPredTile
+// consecutive edges, a lane every 32nd of them: it searches for its row once and
+// walks on.  (A warp per row waits for the longest row: R-MAT of 65,536 vertices
+// 333 us, 36 here.)
+constexpr uint32_t kPredTile = 512;
+__global__ void __launch_bounds__(256) k_pred64(const uint32_t *__restrict__ row, const uint2 *__restrict__ adj,
+                                                const unsigned long long *__restrict__ w64,
+                                                const unsigned long long *__restrict__ dp, uint32_t n, uint32_t m,
+                                                uint32_t src, int32_t *__restrict__ pred) {
     const unsigned lane = threadIdx.x & 31u;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += warps) {
-        const unsigned long long du = dp[u];
-        if (du == kUnreached) continue;
-        const double d = __longlong_as_double((long long)du);
-        for (uint32_t e = row[u] + lane; e < row[u + 1]; e += 32u) {
-            const uint32_t v = adj[e].x;
-            if (v == src) continue;
-            const unsigned long long dv = __ldg(dp + v);
+    const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+    for (unsigned long long t = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) / 32u * kPredTile; t < m;
+         t += warps * kPredTile) {
+        uint32_t u = 0, top = n - 1u;   // the last row that starts at or before the lane's first edge
+        while (u < top) {
+            const uint32_t mid = u + (top - u + 1u) / 2u;
+            if (row[mid] <= t + lane) u = mid;
+            else top = mid - 1u;
+        }
+        unsigned long long du = dp[u];
+        for (unsigned long long e = t + lane; e < min((unsigned long long)m, t + kPredTile); e += 32u) {
+            const uint2 x = adj[e];
+            const unsigned long long w = w64[e];
+            const uint32_t was = u;
+            while (u + 1u < n && row[u + 1u] <= e) ++u;
+            if (u != was) du = dp[u];
+            if (du == kUnreached || x.x == src) continue;
+            const unsigned long long dv = __ldg(dp + x.x);
             if (dv == kUnreached) continue;
-            const double s = __dadd_rn(d, __longlong_as_double((long long)w64[e]));
-            if ((unsigned long long)__double_as_longlong(s) == dv) atomicMin(pred + v, (int32_t)u);
+            const double s = __dadd_rn(__longlong_as_double((long long)du), __longlong_as_double((long long)w));
+            if ((unsigned long long)__double_as_longlong(s) == dv) atomicMin(pred + x.x, (int32_t)u);
         }
     }
 }
@@ -604,7 +618,9 @@ gbs_status launch_run(gbs_graph *g, uint32_t src, const gbs_params *p, void *dis
             k_unpack64<<<eb, tb, 0, s>>>(g->ws.dp, g->n, src, static_cast<unsigned long long *>(dist_dev), pred_dev);
             GBS_CUDA(cudaGetLastError());
             if (pred_dev) {
-                k_pred64<<<g->sms * 8, 256, 0, s>>>(g->d_row, g->d_adj, g->d_w64, g->ws.dp, g->n, src, pred_dev);
+                const uint64_t tiles = (g->m + kPredTile - 1) / kPredTile;   // a warp each
+                k_pred64<<<(int)std::max<uint64_t>(1, std::min<uint64_t>((tiles + 7) / 8, (uint64_t)g->sms * 16)), 256, 0,
+                           s>>>(g->d_row, g->d_adj, g->d_w64, g->ws.dp, g->n, (uint32_t)g->m, src, pred_dev);
                 GBS_CUDA(cudaGetLastError());
             }
         } else if (g->wtype == GBS_WEIGHT_F32) {
