@@ -172,15 +172,22 @@ Workspace carve(unsigned char *base, uint32_t n_cap, uint32_t desc_cap) {
     return w;
 }
 
-// CTAs per group: one group per instance, as long as the groups' distance
-// words (8 bytes per vertex, the target of every random access of a
-// relaxation) fit in L2 together; beyond that, fewer and wider groups.  On
-// R-MAT 22 (33.5 MB per group) 64 groups of 2 CTAs run 2.2x slower than 4
-// groups of 38.
-uint32_t auto_group_ctas(uint32_t count, uint32_t blocks, uint32_t n_cap, size_t l2_bytes) {
-    const size_t per_group = std::max<size_t>(8ull * n_cap, 1);
+// CTAs per group: one group per instance, as long as what the groups gather at
+// random fits in L2 together; beyond that, fewer and wider groups.  Per vertex
+// that is its distance word, and on graphs of many edges a vertex, whose phases
+// touch most vertices, as much again of tags, stamps and lists beside the edges
+// that stream through: ms, 8 -> 16 bytes a vertex, 64 sources of an R-MAT 18
+// 6.95 (64 groups) -> 6.06, 19 13.8 -> 11.4, 20 25.4 -> 23.1, 16 of an R-MAT 21
+// 12.8 -> 11.5, 22 25.8 -> 24.2; but 16 of a 1024^2 grid 14.4 -> 25.5, whose
+// frontiers are thin.  The groups are then evened out over the rounds the
+// instances take, unless a group would be one CTA all the same.
+uint32_t auto_group_ctas(uint32_t count, uint32_t blocks, uint32_t n_cap, uint64_t m_cap, size_t l2_bytes) {
+    const size_t per_group = std::max<size_t>((m_cap > 8ull * n_cap ? 16ull : 8ull) * n_cap, 1);
     const size_t fit = std::max<size_t>((l2_bytes + per_group / 2) / per_group, 1);   // rounded
-    const uint32_t groups = (uint32_t)std::min<size_t>({fit, (size_t)std::max(count, 1u), (size_t)blocks});
+    uint32_t groups = (uint32_t)std::min<size_t>({fit, (size_t)std::max(count, 1u), (size_t)blocks});
+    const uint32_t rounds = (std::max(count, 1u) + groups - 1u) / groups;
+    const uint32_t even = (std::max(count, 1u) + rounds - 1u) / rounds;
+    if (blocks / even >= 2u) groups = even;
     return std::max(1u, blocks / groups);
 }
 
@@ -194,7 +201,7 @@ gbs_status build_plan(gbs_plan *p, const gbs_batch_params *bp, int sms, uint32_t
     int dev = 0, l2 = 0;
     GBS_CUDA(cudaGetDevice(&dev));
     GBS_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-    uint32_t gc = (bp && bp->group_ctas) ? bp->group_ctas : auto_group_ctas(p->count, max_blocks, n_cap, (size_t)l2);
+    uint32_t gc = (bp && bp->group_ctas) ? bp->group_ctas : auto_group_ctas(p->count, max_blocks, n_cap, m_cap, (size_t)l2);
     gc = std::min(gc, max_blocks);
     uint32_t groups = std::min(max_blocks / gc, p->count);
     uint32_t desc_cap = 0;

@@ -437,7 +437,7 @@ typedef struct gbs_batch_params {
                               instance's delta; +INFINITY: no split (every edge
                               light) */
     uint32_t group_ctas;   /* CTAs per group (0: one group per instance while the
-                              groups' distance words, 8 bytes per vertex each,
+                              groups' working sets, 8 to 16 bytes per vertex each,
                               fit in L2; fewer and wider groups beyond) */
     uint32_t flags;        /* GBS_F_NO_SOLO, GBS_F_NO_FUSE */
     uint32_t wait_limit_ms;
