@@ -362,8 +362,13 @@ __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &
         } else if (kind[j] == 2u) {
             r[j] = atomicMin(a.ws.tag + v[j], nb[j]);
         } else if (kind[j] == 3u) {
-            atomicMin(t.c.at(kCPmin + t.pend_sel), nb[j]);
+            // the pending minimum drops only for a vertex that is pending: one
+            // whose later improvement, by another warp, reached its tag first
+            // is in the ring.  A minimum without an entry would stay behind
+            // the window and pull it back at the next pending vertex, where
+            // ring lists stand for other buckets and their vertices are lost
             r[j] = atomicMin(a.ws.tag + v[j], kTagPending);
+            if (r[j] >= kTagPending) atomicMin(t.c.at(kCPmin + t.pend_sel), nb[j]);
             // the pending minimum and tag steer the next decision and the
             // next re-bucketing, which a phase run by one CTA reaches through
             // __syncthreads alone: it does not wait for a global reduction

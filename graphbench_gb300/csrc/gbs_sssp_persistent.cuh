@@ -796,7 +796,7 @@ __device__ inline void control_step(const SsspArgs &a, const Uniform &U, bool wa
         const uint32_t pm = ps2 ? pm1 : pm0;
         if (pcnt > 0 && pm <= found) {
             next = kPhPending;
-            nb = pm;
+            nb = max(pm, scan_from);   // the window never moves back
         } else if (found != 0xFFFFFFFFu) {
             next = kPhLightFirst;
             nb = found;
