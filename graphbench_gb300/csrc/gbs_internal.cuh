@@ -11,7 +11,8 @@
 //                     float32 bit patterns order like the values, so one 64-bit
 //                     atomicMin updates distance and predecessor together and
 //                     keeps the smallest predecessor among equal distances.
-//   tag[n]    uint32  smallest bucket the vertex was queued for (ring dedup)
+//   tag[n]    uint32  whether the vertex is on the pending list (kTagPending), or
+//                     the bucket it left it for
 //   fst[n]    uint32  frontier stamp (dedup inside one light sub-phase)
 //   hst[n]    uint32  heavy-round stamp (a vertex's heavy edges are described
 //                     once per heavy round)

@@ -319,8 +319,18 @@ __device__ __forceinline__ bool edge_sum(typename Arith<WT>::D du, typename Arit
 // improved target joins.  Every step issues its U atomics before using any
 // result, so they are in flight together:
 //   1. packed (dist << 32 | pred) atomicMin: did the distance drop?
-//   2. dedup: same bucket -> frontier stamp; window -> smallest queued
-//      bucket (tag); beyond the window -> pending (tag = kTagPending)
+//   2. dedup: same bucket -> frontier stamp; window -> the bucket of the old
+//      distance: whoever moved the vertex into the new bucket first queued it,
+//      and the 64-bit atomicMin orders the moves, so a vertex whose bucket did
+//      not change is in that bucket's list already (or on the pending list,
+//      which is re-bucketed before its smallest bucket starts); beyond the
+//      window -> pending (tag).  A tag only says whether a vertex is pending: it
+//      is lowered, without waiting for the result, when a vertex that may be
+//      pending is queued elsewhere.  Asking the tag for every target in the
+//      window was a third dependent round trip to L2 per improvement, and
+//      scans read it again: R-MAT of 4 M edges 1505 -> 1397 us of kernel time
+//      without, 64 sources of a 256 k-edge R-MAT 6.13 -> 5.59 ms, 16 of an
+//      R-MAT 22 23.3 -> 20.9 ms; grids, bound by their chain of phases, the same.
 template <int WT, int U>
 __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &t, const bool (&cand)[U],
                                               const uint32_t (&v)[U], const uint32_t (&uo)[U],
@@ -339,12 +349,18 @@ __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &
         kind[j] = !dec ? 0u
                 : nb[j] < t.cur_hi ? 1u
                 : (unsigned long long)nb[j] < (unsigned long long)t.W + kNB ? 2u : 3u;
+        if ((kind[j] == 1u || kind[j] == 2u) && old[j] != kUnreached) {
+            const uint32_t ob = bucket_of<WT>(dist_of<WT>(old[j]), a);
+            // pending entries come from beyond a window of kNB buckets; one that
+            // stays in its bucket stays pending, unless it is relaxed right away
+            if (ob >= (uint32_t)kNB && (kind[j] == 1u || ob != nb[j])) atomicMin(a.ws.tag + v[j], nb[j]);
+            if (kind[j] == 2u && ob == nb[j]) kind[j] = 0u;   // in that list already
+        }
     }
 #pragma unroll
     for (int j = 0; j < U; ++j) {
         r[j] = 0;
         if (kind[j] == 1u) {
-            atomicMin(a.ws.tag + v[j], nb[j]);
             bool kept = false;
             if constexpr (WT != kWF64) {
                 if (t.fuse && loc.v == kNoLocal) {
@@ -359,8 +375,6 @@ __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &
             } else {
                 r[j] = atomicExch(a.ws.fst + v[j], t.stamp_next);
             }
-        } else if (kind[j] == 2u) {
-            r[j] = atomicMin(a.ws.tag + v[j], nb[j]);
         } else if (kind[j] == 3u) {
             // the pending minimum drops only for a vertex that is pending: one
             // whose later improvement, by another warp, reached its tag first
@@ -383,7 +397,7 @@ __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &
             q[j] = 0;
             prefetch_l2(a.g.row + v[j]);   // the next frontier scan reads it
         }
-        else if (kind[j] == 2u && r[j] > nb[j]) q[j] = 1 + (int)(nb[j] % kNB);
+        else if (kind[j] == 2u) q[j] = 1 + (int)(nb[j] % kNB);
         else if (kind[j] == 3u && r[j] == kTagInit) q[j] = kNB + 1;
     }
 }

@@ -190,7 +190,7 @@ __device__ __forceinline__ void fuse_drain(const SsspArgs &a, const Targets &t, 
 }
 
 // One lane per frontier entry.  vtag != kTagInit keeps only entries whose
-// tag equals it (ring lists may hold entries that moved to a lower bucket).
+// distance is in that bucket (ring lists may hold entries that moved lower).
 // The scan relaxes the light prefix [row, mid) of each row, or the whole row
 // when full.  With a split, a vertex scanned for the first time in the
 // current heavy round also emits descriptors for its heavy edges [mid, end):
@@ -229,13 +229,11 @@ __device__ void scan_frontier(const SsspArgs &a, const Targets &t, const Exec &x
         }
         if (lane < deal && i < count) {
             u = __ldcg(at);
-            // the tag check and the row reads are independent: issue together
-            const uint32_t tg = (vtag == kTagInit) ? vtag : __ldcg(a.ws.tag + u);
             du = dist_of<WT>(__ldcg(a.ws.dp + u));
             const uint32_t r = __ldg(a.g.row + u);
             const uint32_t re = __ldg(a.g.row + u + 1);
             const uint32_t md = full ? re : __ldg(a.ws.mid + u);
-            ok = tg == want;
+            ok = vtag == kTagInit || bucket_of<WT>(du, a) == want;
             s = ok ? r : 0u;
             e = ok ? md : 0u;
             he = ok ? re : 0u;
