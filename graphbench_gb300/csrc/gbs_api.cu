@@ -818,9 +818,10 @@ gbs_status gbs_graph_create(uint32_t n, uint64_t m, const uint64_t *row_offsets,
     gbs_status st = check_csr(n, m, row_offsets, cols, weights, wtype, true);
     if (st != GBS_OK) return st;
     // checked and sorted on the device; on the host where its arrays do not
-    // fit beside the graph
+    // fit beside the graph, or where there is no device: a malformed graph is
+    // reported as such there too, before the missing device is
     st = graph_from_host(n, m, row_offsets, cols, weights, wtype, out);
-    if (st != GBS_ERR_NO_MEMORY) return st;
+    if (st != GBS_ERR_NO_MEMORY && st != GBS_ERR_CUDA) return st;
     std::vector<uint32_t> row32;
     std::vector<uint2> adj;
     double max_w = 0.0;
