@@ -301,8 +301,8 @@ def arm_betweenness(gb, g, hg, srcs, cpu: bool, n_src: int = 16):
            "sources": k, "ms_per_source": st["device_ms"] / k,
            "sssp_ms_per_source": st["sssp_ms"] / k, "dag_ms_per_source": st["dag_ms"] / k,
            "max_levels": st["max_levels"], "tight_edges_per_source": st["tight_edges"] / k,
-           "path": "gbs_bc (C ABI): batched gbs_plan_sources launches of up to 64 sources, then one "
-                   "cooperative bc_dag launch per source; result accumulated on the device"}
+           "path": "gbs_bc (C ABI): batched gbs_plan_sources launches of up to 64 sources, then "
+                   "cooperative DAG launches over groups of sources; result accumulated on the device"}
     if cpu:
         import oracle
         one = [int(srcs[n_src % len(srcs)])]
