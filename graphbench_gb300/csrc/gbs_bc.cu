@@ -785,7 +785,7 @@ __device__ __forceinline__ void dag_passes(const BcArgs &a, uint32_t rank, uint3
     unsigned long long tight_n = 0;
     using S = State<WT, Word>;
     for (uint32_t u = rank * blockDim.x + threadIdx.x; u < a.n; u += nblocks * blockDim.x) {
-        if (!a.bc) a.delta[u] = 0.0;   // k_bc_sum reads it; the source and unreached vertices keep it
+        a.delta[u] = 0.0;   // k_bc_sum reads it; vertices that join no level keep it
         if (__ldg(static_cast<const typename S::T *>(a.state) + u) != S::kNone) a.sigma[u] = u == a.source ? 1ull : 0ull;
     }
     count_words<WT, Word>(a, gwarp, nwarps, tight_n);
@@ -997,8 +997,6 @@ gbs_status ensure_groups(gbs_graph *g, BcState *b, uint32_t groups) {
     GBS_CUDA(cudaMalloc(&b->vw_part, sizeof(double) * vw * G));
     GBS_CUDA(cudaMalloc(&b->mask, sizeof(uint32_t) * b->mask_words * G));
     GBS_CUDA(cudaMalloc(&b->ctl, sizeof(BcCtl) * G));
-    // in-degrees return to zero at the end of every FORWARD pass
-    GBS_CUDA(cudaMemsetAsync(b->indeg, 0, sizeof(uint32_t) * n * G, g->stream));
     b->groups = groups;
     return GBS_OK;
 }
@@ -1160,6 +1158,10 @@ gbs_status run_bc(gbs_graph *g, const uint32_t *sources, uint32_t k, const gbs_p
             GBS_CUDA(cudaEventRecord(e0, s));
             GBS_CUDA(cudaMemsetAsync(b->ctl, 0, sizeof(BcCtl) * here, s));
             GBS_CUDA(cudaMemsetAsync(b->mask, 0, sizeof(uint32_t) * b->mask_words * here, s));
+            // FORWARD counts in-degrees down to zero, but not those of vertices
+            // whose tight edges form a cycle (float weights that a sum absorbs),
+            // nor those left by a launch that ran out of its wait limit
+            GBS_CUDA(cudaMemsetAsync(b->indeg, 0, sizeof(uint32_t) * n * here, s));
             GBS_CUDA(cudaLaunchCooperativeKernel(bc_kernel(g->wtype, word, here > 1), dim3(ctas * here), dim3(kBcTPB),
                                                  here > 1 ? many : one, 0, s));
             if (groups > 1)
