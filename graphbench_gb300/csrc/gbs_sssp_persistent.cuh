@@ -101,14 +101,14 @@ __device__ __forceinline__ uint32_t pack_state(const Uniform &N) {
            ((N.span & 0xFFu) << 24);
 }
 
-// Writes a warp's descriptors.  Lane l owns descriptors [excl_l, excl_l + n_l)
-// of the warp's `total` (exclusive prefix excl); its descriptor c covers edges
-// [s_l + c kDescEdges, min(e_l, s_l + (c + 1) kDescEdges)) of row u_l and
-// carries y_l.  The 32 lanes write them together, 32 per round (each finds the
+// Writes a warp's descriptors, those of them that a list of `cap` holds.  Lane l
+// owns descriptors [excl_l, excl_l + n_l) of the warp's `total` (exclusive prefix
+// excl); its descriptor c covers edges [s_l + c kDescEdges, min(e_l, s_l + (c +
+// 1) kDescEdges)) of row u_l and carries y_l.  The 32 lanes write them together, 32 per round (each finds the
 // owning lane by a binary search over excl), so the hundreds of descriptors
 // of a hub row do not queue on its lane.
-__device__ __forceinline__ void write_descs(uint4 *out, uint32_t base, uint32_t total, uint32_t excl, uint32_t u,
-                                            uint32_t y, uint32_t s, uint32_t e) {
+__device__ __forceinline__ void write_descs(uint4 *out, uint32_t cap, uint32_t base, uint32_t total, uint32_t excl,
+                                            uint32_t u, uint32_t y, uint32_t s, uint32_t e) {
     const unsigned FULL = 0xffffffffu;
     const unsigned lane = lane_id();
     for (uint32_t k0 = 0; k0 < total; k0 += 32u) {
@@ -122,18 +122,28 @@ __device__ __forceinline__ void write_descs(uint4 *out, uint32_t base, uint32_t 
         const uint32_t ou = __shfl_sync(FULL, u, own), oy = __shfl_sync(FULL, y, own);
         const uint32_t os = __shfl_sync(FULL, s, own), oe = __shfl_sync(FULL, e, own);
         const uint32_t ox = __shfl_sync(FULL, excl, own);
-        if (k < total) {
+        if (k < total && base + k < cap) {
             const uint32_t cs = os + (k - ox) * kDescEdges;
             out[base + k] = make_uint4(ou, oy, cs, min(oe, cs + kDescEdges));
         }
     }
 }
 
+// The vertices u of a warp whose rows found no room in the descriptor list join
+// the next frontier (lanes with a stamp).  Out of line: it takes no registers
+// from the scans.
+__device__ __noinline__ inline void no_room(const SsspArgs &a, uint32_t fq_next, uint32_t *fq_cnt, uint32_t stamp,
+                                            uint32_t u) {
+    warp_append(a.ws.fq + (size_t)fq_next * a.g.n, fq_cnt, a.g.n,
+                stamp != 0u && atomicExch(a.ws.fst + u, stamp) != stamp, u, a.ws.ctl);
+}
+
 // ------------------------------------------------------------------- SCAN
 // Warp-collective: every lane's row range [s, e) of source u (distance bits
 // du; an empty range for a lane without one).  Rows longer than inline_max
-// become descriptors, reserved with one atomic per warp; the others are
-// relaxed by this warp now.  Edges handed to EDGES add to my_edges.
+// become descriptors, reserved with one atomic per warp, or wait for the next
+// frontier scan where their list is full; the others are relaxed by this warp
+// now.  Edges handed to EDGES add to my_edges.
 template <int WT>
 __device__ __forceinline__ void scan_rows(const SsspArgs &a, const Targets &t, uint32_t u,
                                           typename Arith<WT>::D du, uint32_t s, uint32_t e, uint32_t &my_edges,
@@ -153,13 +163,13 @@ __device__ __forceinline__ void scan_rows(const SsspArgs &a, const Targets &t, u
         uint32_t dbase = 0;
         if (lane == 31) dbase = atomicAdd(t.c.at(kCDesc), total);
         dbase = __shfl_sync(FULL, dbase, 31);
-        if (dbase + total <= a.ws.desc_cap) {
-            // float64 distances do not fit the descriptor: the relaxation
-            // reads dp[u] again (a fresher value is as valid)
-            write_descs(a.ws.desc, dbase, total, incl - nd, u, WT == kWF64 ? 0u : (uint32_t)du, s, e);
-        } else if (lane == 31) {
-            atomicExch(&a.ws.ctl->error, (uint32_t)kErrCapacity);
-        }
+        // float64 distances do not fit the descriptor: the relaxation
+        // reads dp[u] again (a fresher value is as valid)
+        write_descs(a.ws.desc, a.ws.desc_cap, dbase, total, incl - nd, u, WT == kWF64 ? 0u : (uint32_t)du, s, e);
+        // the list holds every row of a scan once, but fusion scans a vertex
+        // again for each improvement that a lane kept
+        if (dbase + total > a.ws.desc_cap)
+            no_room(a, t.fq_next, t.c.at(kCFq + t.fq_next), nd ? t.stamp_next : 0u, u);
         my_edges += nd ? len : 0u;
     }
     relax_group<WT>(a, t, u, du, s, nd ? 0u : len, nc, imp, loc);
@@ -258,7 +268,7 @@ __device__ void scan_frontier(const SsspArgs &a, const Targets &t, const Exec &x
                 if (lane == 31) hbase = atomicAdd(t.c.at(kCHdesc), htotal);
                 hbase = __shfl_sync(FULL, hbase, 31);
                 if (hbase + htotal <= a.ws.desc_cap) {
-                    write_descs(a.ws.hdesc, hbase, htotal, hincl - hn, u, 0u, e, he);
+                    write_descs(a.ws.hdesc, a.ws.desc_cap, hbase, htotal, hincl - hn, u, 0u, e, he);
                 } else if (lane == 31) {
                     atomicExch(&ctl->error, (uint32_t)kErrCapacity);
                 }
@@ -463,8 +473,27 @@ __device__ void finish_instance(const SsspArgs &a, const Exec &x, uint32_t &imp)
     imp = 0;
 }
 
-// Runs the phase U.phase with executor x (grid or one CTA).
-template <int WT>
+// The ring lists of every base bucket that the bucket spans (at most
+// kMergeMax): their entries, and lane j's exclusive prefix of the sizes.
+__device__ __forceinline__ uint32_t ring_lists(const SsspArgs &a, const Uniform &U, const Ctrs &c, uint32_t &excl) {
+    const unsigned lane = lane_id();
+    const uint32_t len = lane < U.span ? min(ld_relaxed_any(c.at(kCRing + (U.b + lane) % kNB)), a.g.n) : 0u;
+    uint32_t incl = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)lane >= o) incl += y;
+    }
+    excl = incl - len;
+    return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// Runs the phase U.phase with executor x (grid or one CTA).  Float32 single runs
+// call the scan from one place: from three they spill 172 bytes a thread instead
+// of 48 (1024^2 grid 16.3 ms instead of 13.6).  The others spill the same either
+// way and are up to 7 % faster with three (float64 300^2 grid 5.34 against 5.73
+// ms, 64 sources of an R-MAT 18 5.65 against 5.95).
+template <int WT, bool Batch>
 __device__ void run_phase(const SsspArgs &a, const Uniform &U, const Exec &x, WarpScratch *scr,
                           uint32_t &imp, const Ctrs &c) {
     const uint32_t n = a.g.n;
@@ -483,28 +512,37 @@ __device__ void run_phase(const SsspArgs &a, const Uniform &U, const Exec &x, Wa
     // the input size comes with the decision (U.items); the counters are
     // read only where it was not published
     const bool pub = U.items != kNoItems;
+    constexpr bool kOneSite = WT == kWF32 && !Batch;
+    if constexpr (kOneSite) {
+        if (U.phase == kPhLightFirst || U.phase == kPhLight) {
+            const bool first = U.phase == kPhLightFirst;
+            const uint32_t slot = U.b % kNB, cur = U.epoch % 3u;
+            uint32_t excl = 0u, total;
+            if (first && U.span > 1u) total = ring_lists(a, U, c, excl);
+            else total = min(pub ? U.items : ld_relaxed_any(c.at(first ? kCRing + slot : kCFq + cur)), n);
+            scan_frontier<WT>(a, t, x, first ? a.ws.ring + (size_t)slot * n : a.ws.fq + (size_t)cur * n, total,
+                              first ? U.b : kTagInit, full, U.hround, imp, first ? U.span : 1u, excl);
+            return;
+        }
+    }
     switch (U.phase) {
         case kPhLightFirst:
-            if (U.span == 1u) {
-                const uint32_t cnt = pub ? U.items : ld_relaxed_any(c.at(kCRing + U.b % kNB));
-                scan_frontier<WT>(a, t, x, a.ws.ring + (size_t)(U.b % kNB) * n, min(cnt, n), U.b, full, U.hround, imp);
-            } else {   // the ring lists of every base bucket the bucket spans (at most kMergeMax)
-                const unsigned lane = lane_id();
-                const uint32_t len = lane < U.span ? min(ld_relaxed_any(c.at(kCRing + (U.b + lane) % kNB)), n) : 0u;
-                uint32_t incl = len;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if ((int)lane >= o) incl += y;
+            if constexpr (!kOneSite) {
+                if (U.span == 1u) {
+                    const uint32_t cnt = pub ? U.items : ld_relaxed_any(c.at(kCRing + U.b % kNB));
+                    scan_frontier<WT>(a, t, x, a.ws.ring + (size_t)(U.b % kNB) * n, min(cnt, n), U.b, full, U.hround, imp);
+                } else {
+                    uint32_t excl;
+                    const uint32_t total = ring_lists(a, U, c, excl);
+                    scan_frontier<WT>(a, t, x, nullptr, total, U.b, full, U.hround, imp, U.span, excl);
                 }
-                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-                scan_frontier<WT>(a, t, x, nullptr, total, U.b, full, U.hround, imp, U.span, incl - len);
             }
             break;
         case kPhLight:
-            scan_frontier<WT>(a, t, x, a.ws.fq + (size_t)(U.epoch % 3u) * n,
-                              min(pub ? U.items : ld_relaxed_any(c.at(kCFq + U.epoch % 3u)), n), kTagInit, full,
-                              U.hround, imp);
+            if constexpr (!kOneSite)
+                scan_frontier<WT>(a, t, x, a.ws.fq + (size_t)(U.epoch % 3u) * n,
+                                  min(pub ? U.items : ld_relaxed_any(c.at(kCFq + U.epoch % 3u)), n), kTagInit, full,
+                                  U.hround, imp);
             break;
         case kPhHeavy:
             relax_heavy<WT>(a, t, x, min(pub ? U.items : ld_relaxed_any(c.at(kCHdesc)), a.ws.desc_cap), imp);
@@ -1064,7 +1102,7 @@ __device__ __forceinline__ void barrier_and_decide(const SsspArgs &a, Uniform &U
                 __threadfence();
                 __syncthreads();
             }
-            run_phase<WT>(a, U, cta_exec(), scr, imp, Ctrs{s_cnt, 1u});
+            run_phase<WT, Batch>(a, U, cta_exec(), scr, imp, Ctrs{s_cnt, 1u});
             if (U.phase == kPhPending) __threadfence();
             // the decision is taken by this CTA: __syncthreads makes every
             // global access of the phase (the fire-and-forget tag and pend_min
@@ -1148,7 +1186,7 @@ __global__ void __launch_bounds__(kTPB, 1) sssp_persistent(SsspArgs a) {
     U.t0 = globaltimer();
     uint32_t imp = 0;
     while (U.phase != kPhDone) {
-        run_phase<WT>(a, U, group_exec(a), scr, imp, global_ctrs(ctl));
+        run_phase<WT, false>(a, U, group_exec(a), scr, imp, global_ctrs(ctl));
         barrier_and_decide<WT, false>(a, U, scr, imp);
     }
     for (int o = 16; o > 0; o >>= 1) imp += __shfl_down_sync(0xffffffffu, imp, o);
@@ -1211,7 +1249,7 @@ __global__ void __launch_bounds__(kTPB, 1) sssp_batch(SsspArgs base, const Works
             loaded = U.inst;
             U.t0 = globaltimer();   // the run-time limit applies per instance
         }
-        run_phase<WT>(s_a, U, group_exec(s_a), scr, imp, global_ctrs(ctl));
+        run_phase<WT, true>(s_a, U, group_exec(s_a), scr, imp, global_ctrs(ctl));
         barrier_and_decide<WT, true>(s_a, U, scr, imp);
     }
     if (group_rank(s_a) == 0 && threadIdx.x == 0) {
