@@ -10,9 +10,11 @@
 
 namespace gbs {
 
-// Sets the thread's last-error message and returns the status.
+// Sets the thread's last-error message and returns the status.  A CUDA error that is reported here leaves nothing pending in the runtime:
+// successful calls do not clear it, so the next launch check would read it.
 inline gbs_status fail(gbs_status s, const std::string &msg) {
     set_last_error(msg.c_str());
+    if (s == GBS_ERR_CUDA || s == GBS_ERR_NO_MEMORY) cudaGetLastError();
     return s;
 }
 

@@ -43,6 +43,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "gbs_host.hpp"
@@ -412,13 +413,21 @@ __global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, 
 // otherwise.  Calls beyond kMaxBlock do not reserve: freeing each buffer when
 // it is done keeps their peak lower.
 constexpr size_t kMaxBlock = 8ull << 30;
+// Failure-path tests: bytes one call may hold on this thread (gbs_test_buffer_limit).
+thread_local size_t t_buffer_limit = SIZE_MAX;
 struct Bufs {
-    std::vector<void *> own;
+    std::vector<std::pair<void *, size_t>> own;
     char *block = nullptr;
-    size_t cap = 0, used = 0;
+    size_t cap = 0, used = 0, held = 0;
+    // past the limit, a size no device has: the runtime's own error
+    cudaError_t alloc(void **p, size_t bytes) {
+        const cudaError_t e = cudaMalloc(p, held + bytes > t_buffer_limit ? (size_t)1 << 62 : bytes);
+        if (e == cudaSuccess) held += bytes;
+        return e;
+    }
     void reserve(size_t bytes) {
         if (block || bytes > kMaxBlock) return;
-        if (cudaMalloc(reinterpret_cast<void **>(&block), bytes) == cudaSuccess) cap = bytes;
+        if (alloc(reinterpret_cast<void **>(&block), bytes) == cudaSuccess) cap = bytes;
         else cudaGetLastError();
     }
     template <typename T> cudaError_t get(T **out, size_t count) {
@@ -429,8 +438,8 @@ struct Bufs {
             return cudaSuccess;
         }
         void *q = nullptr;
-        const cudaError_t e = cudaMalloc(&q, bytes);
-        if (e == cudaSuccess) own.push_back(q);
+        const cudaError_t e = alloc(&q, bytes);
+        if (e == cudaSuccess) own.push_back({q, bytes});
         *out = static_cast<T *>(q);
         return e;
     }
@@ -440,7 +449,10 @@ struct Bufs {
     Mark mark() const { return {used, own.size()}; }
     void reset(Mark m) {
         used = m.used;
-        for (; own.size() > m.own; own.pop_back()) cudaFree(own.back());
+        for (; own.size() > m.own; own.pop_back()) {
+            cudaFree(own.back().first);
+            held -= own.back().second;
+        }
     }
     ~Bufs() {
         reset({0, 0});
@@ -972,6 +984,10 @@ gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const ui
 
 // ===================================================================== C ABI
 extern "C" {
+
+// Not part of the public header: makes a reader or a graph build on this thread
+// that would hold more bytes fail as on a full device (0: no limit).
+void gbs_test_buffer_limit(size_t bytes) { gbs::t_buffer_limit = bytes ? bytes : SIZE_MAX; }
 
 gbs_status gbs_parse_text(const char *bytes, size_t len, int direction, gbs_device_csr **out, gbs_ingest_info *info) {
     if (!out || (len && !bytes)) return gbs::fail(GBS_ERR_INVALID_ARG, "NULL argument");

@@ -1,0 +1,47 @@
+"""A graph whose device build runs out of memory is built on the host, and the
+failed allocation leaves nothing behind: the first solve succeeds."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def limit(gb):
+    f = gb.lib.gbs_test_buffer_limit
+    f.restype, f.argtypes = None, [ctypes.c_size_t]
+    yield f
+    f(0)
+
+
+@pytest.mark.parametrize("wtype", ["u32", "f32", "f64"])
+@pytest.mark.parametrize("scale", [8, 15])          # one CTA, persistent kernel
+def test_host_build_after_a_failed_device_build(wtype, scale, limit, gb, orc):
+    a = gb.gen_rmat(scale, 16, 3, "f32" if wtype == "f32" else "u32")
+    w = a.w / 3.0 if wtype == "f64" else a.w
+    src = int(np.argmax(np.diff(a.row.astype(np.int64))))
+    ref = orc.dijkstra(a.row, a.col, w, src)
+    pred = orc.min_tight_pred(a.row, a.col, w, src, ref)
+    for most in (1, 8 * a.n + 300, 9 * a.m):         # fails at the first buffer, at the columns, in the sort
+        limit(most)
+        with gb.Graph(a.row, a.col, w) as g:
+            limit(0)
+            d, p, _ = g.sssp(src)
+            assert np.array_equal(d, ref) and np.array_equal(p, pred), most
+
+
+def test_other_calls_after_a_failed_build(limit, gb, orc):
+    a = gb.gen_rmat(9, 16, 5)
+    with gb.DeviceCsr.from_arrays(a.row, a.col) as c, gb.Graph.from_host(a) as g:
+        limit(1)
+        with pytest.raises(gb.GbsError) as e:
+            c.graph(gb.W_F32)
+        assert e.value.name == "NO_MEMORY"
+        with pytest.raises(gb.GbsError) as e:
+            gb.DeviceCsr.from_arrays(a.row, a.col)
+        assert e.value.name == "NO_MEMORY"
+        limit(0)
+        d, _, _ = g.sssp(7)
+        assert np.array_equal(d, orc.dijkstra(a.row, a.col, a.w, 7))
