@@ -819,9 +819,10 @@ gbs_status gbs_graph_create(uint32_t n, uint64_t m, const uint64_t *row_offsets,
     if (st != GBS_OK) return st;
     // checked and sorted on the device; on the host where its arrays do not
     // fit beside the graph, or where there is no device: a malformed graph is
-    // reported as such there too, before the missing device is
+    // reported as such there too, before the missing device is.  Any other
+    // failure of a device that is there is the call's
     st = graph_from_host(n, m, row_offsets, cols, weights, wtype, out);
-    if (st != GBS_ERR_NO_MEMORY && st != GBS_ERR_CUDA) return st;
+    if (st != GBS_ERR_NO_MEMORY && !(st == GBS_ERR_CUDA && !gbs_device_available())) return st;
     std::vector<uint32_t> row32;
     std::vector<uint2> adj;
     double max_w = 0.0;

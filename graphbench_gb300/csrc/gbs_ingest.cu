@@ -413,15 +413,19 @@ __global__ void k_row32(const unsigned long long *__restrict__ row, uint32_t n, 
 // otherwise.  Calls beyond kMaxBlock do not reserve: freeing each buffer when
 // it is done keeps their peak lower.
 constexpr size_t kMaxBlock = 8ull << 30;
-// Failure-path tests: bytes one call may hold on this thread (gbs_test_buffer_limit).
+// Failure-path tests: bytes one call may hold on this thread, and whether it fails
+// beyond them for want of memory (gbs_test_buffer_limit).
 thread_local size_t t_buffer_limit = SIZE_MAX;
+thread_local bool t_limit_is_memory = true;
 struct Bufs {
     std::vector<std::pair<void *, size_t>> own;
     char *block = nullptr;
     size_t cap = 0, used = 0, held = 0;
-    // past the limit, a size no device has: the runtime's own error
+    // memory that runs out is a size no device has: the runtime's own error
     cudaError_t alloc(void **p, size_t bytes) {
-        const cudaError_t e = cudaMalloc(p, held + bytes > t_buffer_limit ? (size_t)1 << 62 : bytes);
+        const bool over = held + bytes > t_buffer_limit;
+        if (over && !t_limit_is_memory) return cudaErrorUnknown;
+        const cudaError_t e = cudaMalloc(p, over ? (size_t)1 << 62 : bytes);
         if (e == cudaSuccess) held += bytes;
         return e;
     }
@@ -986,8 +990,12 @@ gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const ui
 extern "C" {
 
 // Not part of the public header: makes a reader or a graph build on this thread
-// that would hold more bytes fail as on a full device (0: no limit).
-void gbs_test_buffer_limit(size_t bytes) { gbs::t_buffer_limit = bytes ? bytes : SIZE_MAX; }
+// that would hold more bytes fail as on a full device, or (memory 0) with
+// another error (bytes 0: no limit).
+void gbs_test_buffer_limit(size_t bytes, int memory) {
+    gbs::t_buffer_limit = bytes ? bytes : SIZE_MAX;
+    gbs::t_limit_is_memory = memory != 0;
+}
 
 gbs_status gbs_parse_text(const char *bytes, size_t len, int direction, gbs_device_csr **out, gbs_ingest_info *info) {
     if (!out || (len && !bytes)) return gbs::fail(GBS_ERR_INVALID_ARG, "NULL argument");

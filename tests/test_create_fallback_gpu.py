@@ -11,9 +11,9 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture
 def limit(gb):
     f = gb.lib.gbs_test_buffer_limit
-    f.restype, f.argtypes = None, [ctypes.c_size_t]
-    yield f
-    f(0)
+    f.restype, f.argtypes = None, [ctypes.c_size_t, ctypes.c_int]
+    yield lambda most, memory=1: f(most, memory)
+    f(0, 1)
 
 
 @pytest.mark.parametrize("wtype", ["u32", "f32", "f64"])
@@ -45,3 +45,16 @@ def test_other_calls_after_a_failed_build(limit, gb, orc):
         limit(0)
         d, _, _ = g.sssp(7)
         assert np.array_equal(d, orc.dijkstra(a.row, a.col, a.w, 7))
+
+
+def test_other_failures_are_reported(limit, gb, orc):
+    """Only a full device, or none, sends a build to the host."""
+    a = gb.gen_rmat(9, 16, 5)
+    for most in (1, 9 * a.m):
+        limit(most, 0)
+        with pytest.raises(gb.GbsError) as e:
+            gb.Graph.from_host(a)
+        assert e.value.name == "CUDA"
+    limit(0)
+    with gb.Graph.from_host(a) as g:
+        assert np.array_equal(g.sssp(7)[0], orc.dijkstra(a.row, a.col, a.w, 7))
