@@ -700,7 +700,7 @@ gbs_status run_sssp(gbs_graph *g, uint32_t src, const gbs_params *p, void *dist_
                     gbs_stats *stats) {
     // without an output the caller wants the state words of the workspace
     if ((dist_dev || pred_dev) && small_call(g, p))
-        return small_run(g, src, dist_dev, pred_dev, !(p && (p->flags & GBS_F_NO_STATS)), stats);
+        return small_run(g, src, dist_dev, pred_dev, p ? p->light : -1.0, !(p && (p->flags & GBS_F_NO_STATS)), stats);
     const bool learned = p && (p->flags & GBS_F_LEARNED);
     if (!learned) return launch_run(g, src, p, dist_dev, pred_dev, stats, false, nullptr);
     if (!g->d_mlp) return fail(GBS_ERR_INVALID_ARG, "GBS_F_LEARNED: no controller set (gbs_graph_set_controller)");

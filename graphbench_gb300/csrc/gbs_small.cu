@@ -470,7 +470,8 @@ gbs_status small_launch(bool f32, const SmallShape &shape, uint32_t grid, const 
     return GBS_OK;
 }
 
-gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, bool want_stats, gbs_stats *stats) {
+gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, double light, bool want_stats,
+                     gbs_stats *stats) {
     if (src >= g->n) return fail(GBS_ERR_INVALID_ARG, "source out of range");
     const SmallShape shape = small_shape(g->n, g->m);
     const bool f32 = g->wtype == GBS_WEIGHT_F32;
@@ -479,7 +480,7 @@ gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, bool
         GBS_CUDA(cudaFuncSetAttribute(kernel_of(f32, false), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kSmallBytes));
     }
-    const Resolved r = resolve_schedule(g->wtype, g->max_w, g->n, g->m, 0.0, -1.0);
+    const Resolved r = resolve_schedule(g->wtype, g->max_w, g->n, g->m, 0.0, light);
     const double wide = r.delta * width_scale(g->n, g->m, false);
     uint32_t width;
     if (f32) {

@@ -20,13 +20,15 @@ SmallShape small_shape(uint32_t n, uint64_t m);
 // uint32) no path sum that could pass 2^32 - 1.
 bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, bool batched);
 
-// Whether this call runs on one CTA: a small graph and no knob set (a delta
-// that resolves to the default width is the default).
+// Whether this call runs on one CTA: a small graph and no knob set that would
+// shape the run (a delta that resolves to the default width is the default; the
+// light bound shapes only runs that set full_items, as in the persistent kernel).
 bool small_call(const gbs_graph *g, const gbs_params *p);
 
 // One source of a resident graph: dist / pred (device or mapped host memory,
-// either may be null) and the statistics, in one launch on g->stream.
-gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, bool want_stats,
+// either may be null) and the statistics, in one launch on g->stream.  `light`:
+// the caller's bound, for the statistics.
+gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, double light, bool want_stats,
                      gbs_stats *stats);
 
 // Instances of a plan: one CTA per instance, taken from `queue` until `count`

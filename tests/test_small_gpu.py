@@ -104,3 +104,17 @@ def test_small_plans(wtype, gb, orc):
             assert np.array_equal(dist[i], ref), i
             assert np.array_equal(pred[i], orc.min_tight_pred(h.row, h.col, h.w, int(sr[i]), ref)), i
             assert st["per_instance"][i]["reached"] == int(np.sum(pred[i] >= 0))
+
+
+@pytest.mark.parametrize("wtype", ["u32", "f32"])
+def test_small_light_bound(wtype, gb, orc):
+    """A light bound alone keeps the one-CTA path (no run without full_items
+    splits) and is reported as the persistent kernel reports it."""
+    a = gb.gen_rmat(9, 16, 8, wtype)
+    ref = orc.dijkstra(a.row, a.col, a.w, 5)
+    with gb.Graph.from_host(a) as g:
+        for light in (None, 0.0, 3.5, float("inf")):
+            d, _, st = g.sssp(5, light=light)
+            _, _, s2 = g.sssp(5, light=light, solo_entries=512)
+            assert st["blocks"] == 1 and s2["blocks"] > 1 and np.array_equal(d, ref)
+            assert st["light_used"] == s2["light_used"], light
