@@ -481,13 +481,14 @@ gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, doub
                                       (int)kSmallBytes));
     }
     const Resolved r = resolve_schedule(g->wtype, g->max_w, g->n, g->m, 0.0, light);
-    const double wide = r.delta * width_scale(g->n, g->m, false);
+    double wide = r.delta * width_scale(g->n, g->m, false);
     uint32_t width;
     if (f32) {
         const float w = (float)wide;
         std::memcpy(&width, &w, 4);
     } else {
-        width = (uint32_t)std::min(wide, 4294967295.0);
+        wide = std::min(wide, 4294967295.0);
+        width = (uint32_t)wide;
     }
     GBS_CUDA(cudaEventRecord(g->ev[0], g->stream));
     if (f32)
@@ -514,7 +515,7 @@ gbs_status small_run(gbs_graph *g, uint32_t src, void *dist, int32_t *pred, doub
         stats->buckets = x.buckets;
         stats->phases = stats->solo_phases = x.phases;
         stats->blocks = 1u;
-        stats->delta_used = r.delta;
+        stats->delta_used = wide;
         stats->light_used = r.light;
     }
     return GBS_OK;

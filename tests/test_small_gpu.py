@@ -118,3 +118,20 @@ def test_small_light_bound(wtype, gb, orc):
             _, _, s2 = g.sssp(5, light=light, solo_entries=512)
             assert st["blocks"] == 1 and s2["blocks"] > 1 and np.array_equal(d, ref)
             assert st["light_used"] == s2["light_used"], light
+
+
+@pytest.mark.parametrize("wtype", ["u32", "f32"])
+def test_small_delta_used(wtype, gb):
+    """The width reported is the one that ran: 64 default widths on graphs of at
+    most 8 edges a vertex, 8 on others, and never past the uint32 range."""
+    cases = [(gb.gen_grid(20, 30, 3, wtype), 64), (gb.gen_rmat(9, 16, 8, wtype), 8)]
+    for a, scale in cases:
+        with gb.Graph.from_host(a) as g:
+            base = g.sssp(5, solo_entries=512)[2]["delta_used"]
+            assert g.sssp(5)[2]["delta_used"] == scale * base
+            assert g.sssp(5, delta=base)[2]["delta_used"] == scale * base
+    if wtype == "u32":
+        row, col, w = _csr(2, [(0, 1, 2**31 - 1)], np.uint32)
+        with gb.Graph(row, col, w) as g:
+            d, _, st = g.sssp(0)
+            assert st["delta_used"] == 2**32 - 1 and d.tolist() == [0, 2**31 - 1]
