@@ -312,7 +312,7 @@ template <int WT, typename Src>
 __global__ void __launch_bounds__(256) k_edges(const unsigned long long *__restrict__ row, const uint32_t *__restrict__ col,
                                                const Src *__restrict__ w, uint32_t n, unsigned long long m,
                                                unsigned long long *__restrict__ key, uint32_t *__restrict__ row_of,
-                                               EdgeStats *st) {
+                                               double *__restrict__ part, EdgeStats *st) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
     const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
@@ -356,8 +356,23 @@ __global__ void __launch_bounds__(256) k_edges(const unsigned long long *__restr
     if (lane == 0) {
         if (mx) atomicMax(&st->max_bits, mx);
         if (bad != ~0ull) atomicMin(&st->bad, bad);
-        if (sum != 0.0) atomicAdd(&st->sum, sum);
+        part[warp] = sum;
     }
+}
+
+// The warps' sums of weights, always in one order: the mean weight is an input
+// of the learned controller, and builds of one graph must agree in it.
+constexpr int kSumTPB = 256;
+__global__ void __launch_bounds__(kSumTPB) k_weight_sum(const double *__restrict__ part, uint32_t count, EdgeStats *st) {
+    __shared__ double s[kSumTPB];
+    double x = 0.0;
+    for (uint32_t i = threadIdx.x; i < count; i += kSumTPB) x += part[i];
+    s[threadIdx.x] = x;
+    for (int h = kSumTPB / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if ((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
+    }
+    if (threadIdx.x == 0) st->sum = s[0];
 }
 
 __global__ void k_edge_stats_init(EdgeStats *st) { *st = EdgeStats{~0ull, 0ull, 0.0, 0u, 0u, 0u, 0u}; }
@@ -839,7 +854,11 @@ gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long lon
     EdgeStats *st = nullptr, hs{};
     unsigned long long *key = nullptr, *key_s = nullptr;
     uint32_t *row_of = nullptr, *row32 = nullptr;
+    const int ge = grid_for((m + kEdgeTile - 1) / kEdgeTile * 32, sms);
+    const uint32_t edge_warps = (uint32_t)ge * 8u;   // of 256 threads a block
+    double *part = nullptr;
     ING_CUDA(bufs.get(&st, 1));
+    ING_CUDA(bufs.get(&part, edge_warps));
     ING_CUDA(bufs.get(&key, m));
     ING_CUDA(bufs.get(&key_s, m));
     if (f64) ING_CUDA(bufs.get(&row_of, m));
@@ -850,7 +869,8 @@ gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long lon
     } guard{row32};
     k_edge_stats_init<<<1, 1, 0, s>>>(st);
     k_row32<<<std::max(1, std::min<int>((int)(((unsigned long long)n + 256) / 256), sms * 8)), 256, 0, s>>>(row, n, row32, st);
-    k_edges<WT, Src><<<grid_for((m + kEdgeTile - 1) / kEdgeTile * 32, sms), 256, 0, s>>>(row, col, w, n, m, key, row_of, st);
+    k_edges<WT, Src><<<ge, 256, 0, s>>>(row, col, w, n, m, key, row_of, part, st);
+    k_weight_sum<<<1, kSumTPB, 0, s>>>(part, edge_warps, st);
     ING_CUDA(cudaGetLastError());
     ING_CUDA(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s));
     ING_CUDA(cudaStreamSynchronize(s));

@@ -71,3 +71,29 @@ def test_create_refuses(what, gb):
         with pytest.raises(gb.GbsError) as e:
             gb.Graph(row, col, w.astype(dtype))
         assert e.value.name == "INVALID_ARG" and want in str(e.value)
+
+
+def test_mean_weight_is_reproducible(gb):
+    """Builds of one graph agree in the controller input that holds the mean
+    weight, here half way between two float32 values: the last bit of the sum
+    decides which."""
+    import math
+    n, m = 1 << 12, 1 << 20
+    rng = np.random.default_rng(5)
+    row = np.arange(0, m + 1, m // n, dtype=np.uint64)
+    col = rng.integers(0, n, m).astype(np.uint32)
+    w = rng.random(m)
+    w[0] = 1.0
+    half = m * (0.5 + 2.0 ** -25)                  # float32 values near one half are 2^-24 apart
+    for i in range(1, m):                          # weights moved until the exact sum is m times that
+        gap = half - math.fsum(w)
+        if gap == 0.0:
+            break
+        w[i] = min(max(w[i] + gap, 2.0 ** -20), 1.0 - 2.0 ** -20)
+    assert math.fsum(w) == half
+    seen = set()
+    for _ in range(24):
+        with gb.Graph(row, col, w) as g:
+            g.sssp(1, flags=gb.F_FEATURES)
+            seen.add(float(g.features()[0, 14]))
+    assert len(seen) == 1 and seen <= {0.5, 0.5 + 2.0 ** -24}
