@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) k_pred64(const uint32_t *__restrict__ row
             const uint2 x = adj[e];
             const unsigned long long w = w64[e];
             const uint32_t was = u;
-            while (u + 1u < n && row[u + 1u] <= e) ++u;
+            u = row_at(row, n, u, e);
             if (u != was) du = dp[u];
             if (du == kUnreached || x.x == src) continue;
             const unsigned long long dv = __ldg(dp + x.x);

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) k_edges(const unsigned long long *__restr
             else top = mid - 1u;
         }
         for (unsigned long long e = t + lane; e < min(m, t + kEdgeTile); e += 32u) {
-            while (v + 1u < n && row[v + 1u] <= e) ++v;
+            v = row_at(row, n, v, e);
             const uint32_t c = col[e];
             unsigned long long bits;
             const Src x = w[e];

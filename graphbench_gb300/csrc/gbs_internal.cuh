@@ -340,4 +340,29 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 // Sets the message gbs_last_error returns on the calling thread.
 void set_last_error(const char *msg);
 
+// The last row that starts at or before position e, from row v, which does, on:
+// a few steps, then doubling ones and a search between the last two, so that a
+// long run of empty rows costs its logarithm.  Stays inside the offsets even
+// where they decrease.
+template <typename T>
+__device__ __forceinline__ uint32_t row_at(const T *__restrict__ row, uint32_t n, uint32_t v, unsigned long long e) {
+#pragma unroll 1
+    for (int k = 0; k < 8; ++k) {
+        if (v + 1u >= n || row[v + 1u] > e) return v;
+        ++v;
+    }
+    uint32_t step = 8u;
+    while (step < n - v && row[v + step] <= e) {
+        v += step;
+        step *= 2u;
+    }
+    uint32_t top = step < n - v ? v + step - 1u : n - 1u;
+    while (v < top) {
+        const uint32_t mid = v + (top - v + 1u) / 2u;
+        if (row[mid] <= e) v = mid;
+        else top = mid - 1u;
+    }
+    return v;
+}
+
 }  // namespace gbs

@@ -97,3 +97,28 @@ def test_mean_weight_is_reproducible(gb):
             g.sssp(1, flags=gb.F_FEATURES)
             seen.add(float(g.features()[0, 14]))
     assert len(seen) == 1 and seen <= {0.5, 0.5 + 2.0 ** -24}
+
+
+@pytest.mark.parametrize("wtype", ["u32", "f64"])
+def test_long_runs_of_empty_rows(wtype, gb, orc):
+    """Few edges among many vertices: a build and a float64 solve search past
+    empty rows instead of walking them (they took 400 times as long)."""
+    import time
+    n, m = 1 << 22, 4096
+    rng = np.random.default_rng(8)
+    best = []
+    for most in (n, 64):                          # rows anywhere, rows of 64 edges at the front
+        u, v = np.sort(rng.integers(0, most, m)), rng.integers(0, most, m).astype(np.uint32)
+        row = np.zeros(n + 1, dtype=np.uint64)
+        row[1:] = np.cumsum(np.bincount(u, minlength=n))
+        w = rng.integers(1, 99, m).astype(DT[wtype])
+        times = []
+        for _ in range(4):
+            t = time.perf_counter()
+            with gb.Graph(row, v, w) as g:
+                d, p, _ = g.sssp(int(u[0]))
+            times.append(time.perf_counter() - t)
+        best.append(min(times))
+        ref = orc.dijkstra(row, v, w, int(u[0]))
+        assert np.array_equal(d, ref) and np.array_equal(p, orc.min_tight_pred(row, v, w, int(u[0]), ref))
+    assert best[0] < 3 * best[1], best
