@@ -139,7 +139,7 @@ void free_graph(gbs_graph *g);
 
 // A resident graph from host arrays, checked and sorted on the device
 // (gbs_ingest.cu).  The caller has checked the pointers, n, m and the first and
-// last row offset.  It holds up to 92 bytes per edge beside the graph while it
+// last row offset.  It holds up to 64 bytes per edge beside the graph while it
 // runs (GBS_ERR_NO_MEMORY where they are not there).
 gbs_status graph_from_host(uint32_t n, uint64_t m, const uint64_t *row, const uint32_t *cols, const void *weights,
                            gbs_weight_type wtype, gbs_graph **out);

@@ -842,7 +842,7 @@ __global__ void k_iota(uint32_t *__restrict__ id, unsigned long long m) {
 // messages); else from a device CSR.  gbs_graph_create, checked and sorted by 16
 // host cores -> here, ms: R-MAT 16 6.5 -> 1.1 (float64 10.8 -> 1.7), 20 116 ->
 // 5.6, 22 475 -> 20.
-size_t build_bytes(unsigned long long m, bool f64) { return (f64 ? 60 : 36) * m + (8u << 20); }
+size_t build_bytes(unsigned long long m, bool f64) { return (f64 ? 52 : 36) * m + (8u << 20); }
 
 template <int WT, typename Src>
 gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long long *row, const uint32_t *col, const Src *w,
@@ -919,12 +919,15 @@ gbs_status build_graph(uint32_t n, unsigned long long m, const unsigned long lon
     }
     gbs_graph *g = nullptr;
     if (f64) {
-        // by weight, then by row; key keeps the weights in edge order
-        unsigned long long *a = nullptr, *b = nullptr;
-        ING_CUDA(bufs.get(&a, m));
-        ING_CUDA(bufs.get(&b, m));
+        // by weight, then by row; key keeps the weights in edge order.  The rows'
+        // keys lie where the weights' were, so that a build holds 40 bytes an
+        // edge at most
+        unsigned long long *a = key_s;
+        uint32_t *rk_s = reinterpret_cast<uint32_t *>(key_s);
+        if (hs.unsorted) ING_CUDA(bufs.get(&a, m));
+        else ING_CUDA(bufs.get(&rk_s, m));
         if ((r = sort_pairs<unsigned long long>(hs.unsorted ? key_s : key, a, id0, id1, m, s, bufs)) != GBS_OK) return r;
-        uint32_t *rk = reinterpret_cast<uint32_t *>(a), *rk_s = reinterpret_cast<uint32_t *>(b);
+        uint32_t *rk = reinterpret_cast<uint32_t *>(a);
         k_gather_key<uint32_t><<<gb, 256, 0, s>>>(row_of, id1, m, rk);
         ING_CUDA(cudaGetLastError());
         if ((r = sort_pairs<uint32_t>(rk, rk_s, id1, id0, m, s, bufs, bits_n)) != GBS_OK) return r;

@@ -58,3 +58,22 @@ def test_other_failures_are_reported(limit, gb, orc):
     limit(0)
     with gb.Graph.from_host(a) as g:
         assert np.array_equal(g.sssp(7)[0], orc.dijkstra(a.row, a.col, a.w, 7))
+
+
+@pytest.mark.parametrize("wtype", ["f32", "f64"])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_build_memory(wtype, shuffled, limit, gb, orc):
+    """A build from a device CSR holds at most 40 bytes an edge and the sort's
+    12, whatever the order of the columns."""
+    a = gb.gen_rmat(15, 16, 7)
+    col = a.col
+    if shuffled:
+        rows = np.repeat(np.arange(a.n), np.diff(a.row.astype(np.int64)))
+        col = col[np.lexsort((np.random.default_rng(1).random(a.m), rows))]
+    with gb.DeviceCsr.from_arrays(a.row, col) as c:
+        row, col, w = c.export()
+        limit(52 * a.m + (3 << 20))
+        with c.graph(gb.W_F64 if wtype == "f64" else gb.W_F32) as g:
+            limit(0)
+            d, _, _ = g.sssp(7)
+    assert np.array_equal(d, orc.dijkstra(row, col, w if wtype == "f64" else w.astype(np.float32), 7))
