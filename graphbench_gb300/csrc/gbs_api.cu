@@ -569,7 +569,7 @@ gbs_status launch_run(gbs_graph *g, uint32_t src, const gbs_params *p, void *dis
     a.inline_max = (p && p->inline_edges) ? p->inline_edges : kInlineEdges;
     a.full_items = (p && p->full_items) ? p->full_items : std::max(g->n, kFullItems);
     a.fuse_rounds = (a.flags & GBS_F_NO_FUSE) ? 0u : ((p && p->fuse_rounds) ? p->fuse_rounds : kFuseRounds);
-    merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, learned, a.merge_low, a.merge_drain);
+    merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, learned, a.merge_low, a.merge_ramp, a.merge_drain);
     a.run_ns = a.wait_ns * 16ull;
     a.ctrl = learned ? kCtrlLearned : kCtrlFixed;
     a.span_fixed = 1;

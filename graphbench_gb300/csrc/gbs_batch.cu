@@ -426,7 +426,8 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
         d.delta_u = r.delta_u;
         d.inv_delta_f = r.inv_delta_f;
         d.no_heavy = no_heavy ? 1u : 0u;
-        merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, false, d.merge_low, d.merge_drain);
+        merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, false, d.merge_low, d.merge_ramp,
+                     d.merge_drain);
         d.dist = dist_dev ? static_cast<uint32_t *>(dist_dev) + (size_t)i * g->n : nullptr;
         d.pred = pred_dev ? pred_dev + (size_t)i * g->n : nullptr;
     }
@@ -492,7 +493,8 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
         d.delta_u = rs[i].delta_u;
         d.inv_delta_f = rs[i].inv_delta_f;
         d.no_heavy = nh[i] ? 1u : 0u;
-        merge_limits(pk->wtype, pk->n[i], pk->m[i], pk->max_deg[i], pk->max_w[i], false, d.merge_low, d.merge_drain);
+        merge_limits(pk->wtype, pk->n[i], pk->m[i], pk->max_deg[i], pk->max_w[i], false, d.merge_low, d.merge_ramp,
+                     d.merge_drain);
         d.dist = dist_dev ? static_cast<uint32_t *>(dist_dev) + pk->voff[i] : nullptr;
         d.pred = pred_dev ? pred_dev + pk->voff[i] : nullptr;
         n_cap = std::max(n_cap, pk->n[i]);

@@ -215,6 +215,7 @@ struct InstDesc {
     float inv_delta_f;
     uint32_t no_heavy;
     uint32_t merge_low;     // as SsspArgs.merge_low
+    uint32_t merge_ramp;    // as SsspArgs.merge_ramp
     uint32_t merge_drain;   // as SsspArgs.merge_drain
     uint32_t *dist;
     int32_t *pred;
@@ -260,7 +261,8 @@ struct SsspArgs {
                             // starts relaxes whole rows (no heavy phase)
     uint32_t fuse_rounds;   // bucket fusion rounds per warp in whole-row scans (0: none)
     uint32_t merge_low;     // a bucket takes in the next base buckets while their lists hold at most
-                            // this many entries (0: no such merge; see merge_spans)
+                            // this many entries (0: no such merge; see merge_limits)
+    uint32_t merge_ramp;    // bucket b takes in b / merge_ramp base buckets at most that way (0: no limit)
     uint32_t merge_drain;   // base buckets a bucket takes in while the run drains (0 or 1: none)
     uint32_t merge_whole;   // 1: merged buckets relax whole rows whatever full_items says
     // bucket-width controller

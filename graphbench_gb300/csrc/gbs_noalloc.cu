@@ -251,7 +251,7 @@ extern "C" gbs_status gbs_sssp_noalloc(uint32_t n, uint64_t m, const uint32_t *r
     a.full_items = kFullItems;
     a.fuse_rounds = kFuseRounds;
     // row lengths are not known here: no merge before the run drains
-    merge_limits(wtype, n, m, UINT32_MAX, max_w, false, a.merge_low, a.merge_drain);
+    merge_limits(wtype, n, m, UINT32_MAX, max_w, false, a.merge_low, a.merge_ramp, a.merge_drain);
     a.ctrl = kCtrlFixed;
     a.span_fixed = 1;
     a.wait_ns = 4000ull * 1000000ull;

@@ -74,7 +74,11 @@ inline uint32_t split_full_items(uint32_t n) { return n / 16u > kFullItems ? n /
 //   low    graphs without long rows (road networks, grids, meshes), whose
 //          frontier grows by at most the degree a hop: the next base buckets
 //          while they hold at most kMergeEdges edges (entries x average degree)
-//          together, up to kMergeLow of them
+//          together, up to kMergeLow of them.  Where some row has more than
+//          kMergeFlat edges, bucket b takes in b / kMergeRamp of them at most:
+//          on graphs that spread fast (random graphs: every vertex within some
+//          30 widths) a few entries in a wide bucket reach most of the graph
+//          over bad paths
 //   drain  the run has started 1/16 of the vertices, and either the last
 //          bucket relaxed fewer edges of long rows than it had entries or the
 //          queues shrank over it: what is left are short rows that improve
@@ -89,23 +93,32 @@ inline uint32_t split_full_items(uint32_t n) { return n / 16u > kFullItems ? n /
 // 22 (162,304) 1.97 -> 1.60.  A drain of 8 or 16 base buckets gains a little
 // more (R-MAT 20 0.64, 0.61; 22 1.48, 1.43); a learned run, whose base widths
 // the controller picks, takes up to 32.
+// The ramp (random graphs, ms; no merge in any form, no ramp, a ramp of 4): 64
+// sources of 262,144 vertices and degree 8 (23) 5.10, 6.06, 3.55, degree 4 (16)
+// 3.76, 4.41, 2.48; one source of 1 M vertices and degree 8 1.21, 0.74, 0.66,
+// with unit weights 0.330, 0.353, 0.272, with weights 1 to 3 0.44, 0.52, 0.40;
+// ramps of 1 and 8 instead of 4: 4.67, 3.62 ms and 0.68, 0.72, 0.335, 0.273, 0.42,
+// 0.35.  Lattices and rings of long diameter do not notice it (8.0, 48.3).
 constexpr uint32_t kMergeEdges = 131072u;
 constexpr uint32_t kMergeLow = 16u;
+constexpr uint32_t kMergeFlat = 4u;          // grids, trees, road networks: 0.17 ms a binary tree, 0.30 with the ramp
+constexpr uint32_t kMergeRamp = 4u;
 constexpr uint32_t kMergeDrain = 4u;
 constexpr uint32_t kMergeLearned = 32u;
 constexpr uint32_t kMergeMax = 32u;          // one lane per list of a merged bucket
 
-// The two limits of a graph.  uint32 sums: a vertex of a merged bucket relaxes
+// The limits of a graph.  uint32 sums: a vertex of a merged bucket relaxes
 // its row from a distance that may lie up to the bucket's width above its
 // final one, so a sum could pass 2^32 - 1 that does not in the end; where no
 // path can (n x the largest weight below it) buckets merge, elsewhere not.
 inline void merge_limits(gbs_weight_type wt, uint32_t n, uint64_t m, uint32_t max_deg, double max_w, bool learned,
-                         uint32_t &low, uint32_t &drain) {
-    low = drain = 0u;
+                         uint32_t &low, uint32_t &ramp, uint32_t &drain) {
+    low = ramp = drain = 0u;
     if (n == 0 || (wt == GBS_WEIGHT_U32 && (double)n * max_w >= 4294967295.0)) return;
     if (max_deg <= kInlineEdges) {
         const uint64_t avg = (m + n - 1) / n;
         low = kMergeEdges / (uint32_t)(avg ? avg : 1);
+        ramp = max_deg > kMergeFlat ? kMergeRamp : 0u;
     }
     drain = learned ? kMergeLearned : kMergeDrain;
 }

@@ -704,7 +704,8 @@ __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const
                 const uint32_t y = __shfl_up_sync(FULL, incl, o);
                 if ((int)lane >= o) incl += y;
             }
-            wide = max(wide, (uint32_t)__popc(__ballot_sync(FULL, lane < kMergeLow && incl <= a.merge_low)));
+            const uint32_t most = a.merge_ramp ? min(kMergeLow, nb / a.merge_ramp + 1u) : kMergeLow;
+            wide = max(wide, (uint32_t)__popc(__ballot_sync(FULL, lane < most && incl <= a.merge_low)));
         }
         if (wide > span) {
             span = wide;
@@ -1241,6 +1242,7 @@ __global__ void __launch_bounds__(kTPB, 1) sssp_batch(SsspArgs base, const Works
                 s_a.inv_delta_f = d.inv_delta_f;
                 s_a.no_heavy = d.no_heavy;
                 s_a.merge_low = d.merge_low;
+                s_a.merge_ramp = d.merge_ramp;
                 s_a.merge_drain = d.merge_drain;
                 s_a.dist_out = d.dist;
                 s_a.pred_out = d.pred;

@@ -56,3 +56,24 @@ def test_merged_buckets_same_result(kind, merges, gb, orc):
                 dist, _ = plan.results()
             for i, src in enumerate(srcs):
                 assert np.array_equal(dist[i], orc.dijkstra(row, col, w, src))
+
+
+def _starts(trace):
+    return [r for r in trace if r["kind"] == "scan_bucket"]
+
+
+def test_merges_widen_with_the_distance_on_graphs_that_spread(gb, orc):
+    """Until the run drains, bucket b of a graph with rows of more than four edges
+    takes in b / 4 base buckets; a grid's takes in up to 16 from the start."""
+    row, col, w = _uniform(20000, 6, 7)
+    grid = gb.gen_grid(150, 161, 4, "u32")
+    for r, c, x, ramp in ((row, col, w, True), (grid.row, grid.col, grid.w, False)):
+        n, done, wide = len(r) - 1, 0, False
+        with gb.Graph(r, c, x) as g:
+            d, _, _ = g.sssp(1, flags=gb.F_TRACE)
+            for rec in _starts(g.trace()):
+                if done < n // 16:
+                    wide |= rec["span"] > rec["bucket"] // 4 + 1
+                done += rec["items"]
+        assert wide != ramp
+        assert np.array_equal(d, orc.dijkstra(r, c, x, 1))
