@@ -399,7 +399,7 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
     const Resolved r = schedule_of(params, g->wtype, g->max_w, g->n, g->m);
     const bool no_heavy = r.light_bits >= max_weight_bits(g->wtype, g->max_w);
     const uint32_t *mid = g->d_row + 1;   // no split: the first heavy edge is the row end
-    const bool small = default_plan(params) && small_graph(g->wtype, g->n, g->m, g->max_w, true);
+    const bool small = default_plan(params) && small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, true);
     if (!no_heavy && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * g->n);
         if (e != cudaSuccess) {
@@ -458,7 +458,7 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
         rs[i] = schedule_of(params, pk->wtype, pk->max_w[i], pk->n[i], pk->m[i]);
         nh[i] = rs[i].light_bits >= max_weight_bits(pk->wtype, pk->max_w[i]);
         any_split = any_split || !nh[i];
-        small = small && small_graph(pk->wtype, pk->n[i], pk->m[i], pk->max_w[i], true);
+        small = small && small_graph(pk->wtype, pk->n[i], pk->m[i], pk->max_w[i], 0.0, true);
     }
     if (any_split && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * std::max<uint64_t>(pk->voff[pk->count], 1));

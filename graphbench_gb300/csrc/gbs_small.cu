@@ -53,6 +53,16 @@ constexpr int kSmallTPB = 1024;
 constexpr uint32_t kSmallN = 16384;
 constexpr uint64_t kSmallM = 262144;
 constexpr uint64_t kSmallBatchM = 524288;
+// A graph whose default width is kWideRatio mean weights or more (unit weights,
+// few distinct ones, skewed ones) takes a handful of buckets, which the grid
+// shares well: beyond kSmallWideM edges it is left to the persistent kernel
+// where one CTA is slower.  Persistent kernel before buckets merged -> one CTA,
+// us a call: unit weights, 131,072 edges 88..149 -> 84..119, 196,608 76..101 ->
+// 83..118, 262,144 77..166 -> 99..168; lognormal (sigma 3), 131,072 250..480 ->
+// 190..350, 262,144 247, 261, 458 -> 359, 371, 501.  Weights 1 to 255 at 0.02 to
+// 0.25 widths a mean weight: 262,144 edges 298..864 -> 110..241.
+constexpr uint64_t kSmallWideM = 131072;
+constexpr double kWideRatio = 0.28;
 // Default widths one bucket spans.  Sweeps are short, so wide buckets pay;
 // graphs of few edges a vertex, whose frontier stays thin, hardly repeat work
 // at any width (64 x 100 grid, kernel us: 4 310, 8 254, 64 215).  R-MAT of
@@ -431,7 +441,7 @@ SmallShape small_shape(uint32_t n, uint64_t m) {
 }
 
 bool small_call(const gbs_graph *g, const gbs_params *p) {
-    if (!small_graph(g->wtype, g->n, g->m, g->max_w, false)) return false;
+    if (!small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, false)) return false;
     if (!p) return true;
     if ((p->flags & ~GBS_F_NO_STATS) || p->solo_entries || p->solo_descs || p->inline_edges || p->full_items ||
         p->fuse_rounds)
@@ -440,9 +450,12 @@ bool small_call(const gbs_graph *g, const gbs_params *p) {
                                   resolve_schedule(g->wtype, g->max_w, g->n, g->m, 0.0, -1.0).delta;
 }
 
-bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, bool batched) {
+bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, double mean_w, bool batched) {
     if (n == 0 || n > kSmallN || m > (batched ? kSmallBatchM : kSmallM)) return false;
     if (small_shape(n, m).bytes > kSmallBytes) return false;
+    if (!batched && m > kSmallWideM &&
+        resolve_schedule(wt, max_w, n, m, 0.0, -1.0).delta >= kWideRatio * mean_w)
+        return false;
     if (wt == GBS_WEIGHT_U32) return (double)n * max_w < 4294967295.0;
     return wt == GBS_WEIGHT_F32;
 }

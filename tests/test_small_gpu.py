@@ -135,3 +135,24 @@ def test_small_delta_used(wtype, gb):
         with gb.Graph(row, col, w) as g:
             d, _, st = g.sssp(0)
             assert st["delta_used"] == 2**32 - 1 and d.tolist() == [0, 2**31 - 1]
+
+
+@pytest.mark.parametrize("wtype,weights,m,one", [
+    ("u32", "unit", 131072, True), ("u32", "unit", 131073, False), ("f32", "unit", 262144, True),
+    ("u32", "uniform", 262144, True), ("u32", "uniform", 262145, False),
+    ("f32", "skewed", 131072, True), ("f32", "skewed", 131073, False), ("u32", "zero", 131073, False)])
+def test_small_limit_of_edges(wtype, weights, m, one, gb, orc):
+    """The edge limit, half as large where the default width is a large part of
+    the mean weight (unit float weights have a width of one sixteenth)."""
+    n = 16384
+    rng = np.random.default_rng(m)
+    u, v = np.sort(rng.integers(0, n, m)), rng.integers(0, n, m).astype(np.uint32)
+    row = np.zeros(n + 1, dtype=np.uint64)
+    row[1:] = np.cumsum(np.bincount(u, minlength=n))
+    w = {"unit": np.ones(m), "zero": np.zeros(m), "uniform": rng.integers(1, 256, m), "skewed": rng.lognormal(0, 2, m)}[weights]
+    w = w.astype(np.uint32 if wtype == "u32" else np.float32)
+    with gb.Graph(row, v, w) as g:
+        d, p, st = g.sssp(3)
+    ref = orc.dijkstra(row, v, w, 3)
+    assert (st["blocks"] == 1) == one
+    assert np.array_equal(d, ref) and np.array_equal(p, orc.min_tight_pred(row, v, w, 3, ref))
