@@ -27,7 +27,7 @@ struct gbs_pack {
     int sms = 0;
     std::vector<uint32_t> n;
     std::vector<uint64_t> m;
-    std::vector<double> max_w;
+    std::vector<double> max_w, mean_w;
     std::vector<uint32_t> max_deg;
     std::vector<uint64_t> voff;   // count+1: first vertex of each graph in pack-wide arrays
     std::vector<uint64_t> eoff;   // count+1: first edge of each graph
@@ -327,6 +327,7 @@ gbs_status gbs_pack_create(uint32_t count, const gbs_csr_view *graphs, gbs_weigh
     p->n.resize(count);
     p->m.resize(count);
     p->max_w.resize(count);
+    p->mean_w.assign(count, 0.0);
     p->max_deg.assign(count, 0);
     p->voff.assign(count + 1, 0);
     p->eoff.assign(count + 1, 0);
@@ -356,6 +357,11 @@ gbs_status gbs_pack_create(uint32_t count, const gbs_csr_view *graphs, gbs_weigh
         p->n[i] = v.n;
         p->m[i] = v.m;
         for (uint32_t r = 0; r < v.n; ++r) p->max_deg[i] = std::max(p->max_deg[i], row32[r + 1] - row32[r]);
+        double sum = 0.0;
+        for (uint64_t e = 0; e < v.m; ++e)
+            sum += wtype == GBS_WEIGHT_F32 ? (double)static_cast<const float *>(v.weights)[e]
+                                           : (double)static_cast<const uint32_t *>(v.weights)[e];
+        p->mean_w[i] = v.m ? sum / (double)v.m : 0.0;
         if ((e = cudaMemcpy(p->d_row + p->voff[i] + i, row32.data(), sizeof(uint32_t) * (v.n + 1),
                             cudaMemcpyHostToDevice)) != cudaSuccess ||
             (v.m && (e = cudaMemcpy(p->d_adj + p->eoff[i], adj.data(), sizeof(uint2) * v.m,
@@ -399,7 +405,7 @@ gbs_status gbs_plan_sources(gbs_graph *g, const uint32_t *sources, uint32_t k, c
     const Resolved r = schedule_of(params, g->wtype, g->max_w, g->n, g->m);
     const bool no_heavy = r.light_bits >= max_weight_bits(g->wtype, g->max_w);
     const uint32_t *mid = g->d_row + 1;   // no split: the first heavy edge is the row end
-    const bool small = default_plan(params) && small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, true);
+    const bool small = default_plan(params) && small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, k);
     if (!no_heavy && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * g->n);
         if (e != cudaSuccess) {
@@ -458,7 +464,7 @@ gbs_status gbs_plan_pack(gbs_pack *pk, const uint32_t *sources, const gbs_batch_
         rs[i] = schedule_of(params, pk->wtype, pk->max_w[i], pk->n[i], pk->m[i]);
         nh[i] = rs[i].light_bits >= max_weight_bits(pk->wtype, pk->max_w[i]);
         any_split = any_split || !nh[i];
-        small = small && small_graph(pk->wtype, pk->n[i], pk->m[i], pk->max_w[i], 0.0, true);
+        small = small && small_graph(pk->wtype, pk->n[i], pk->m[i], pk->max_w[i], pk->mean_w[i], pk->count);
     }
     if (any_split && !small) {
         cudaError_t e = cudaMalloc(&p->d_mid, sizeof(uint32_t) * std::max<uint64_t>(pk->voff[pk->count], 1));

@@ -63,6 +63,17 @@ constexpr uint64_t kSmallBatchM = 524288;
 // 0.25 widths a mean weight: 262,144 edges 298..864 -> 110..241.
 constexpr uint64_t kSmallWideM = 131072;
 constexpr double kWideRatio = 0.28;
+// In a plan that holds up to a number of instances, whose CTAs fill the other
+// SMs from there on: kWideStep, one step more beyond kSmallM edges and one more
+// on graphs that are not skewed (largest weight at most kSkew mean weights).
+// Beyond kSmallM edges it holds for every skewed graph.  Persistent kernel before
+// buckets merged -> one CTA, us a plan of 1, 16, 64: unit weights, 4,096 vertices
+// and 262,144 edges 77, 93, 171 -> 128, 128, 130, 520,000 75, 104, 222 -> 236,
+// 247, 247 (152 of them 370 -> 252); lognormal (sigma 2), 262,144 211, 315, 673 ->
+// 305, 329, 343 (sigma 3, 16,384 vertices, 32 of them: 823 -> 605); exponential,
+// 520,000 402, 494, 846 -> 590, 608, 649.
+constexpr uint32_t kWideStep = 32;
+constexpr double kSkew = 4.0;
 // Default widths one bucket spans.  Sweeps are short, so wide buckets pay;
 // graphs of few edges a vertex, whose frontier stays thin, hardly repeat work
 // at any width (64 x 100 grid, kernel us: 4 310, 8 254, 64 215).  R-MAT of
@@ -441,7 +452,7 @@ SmallShape small_shape(uint32_t n, uint64_t m) {
 }
 
 bool small_call(const gbs_graph *g, const gbs_params *p) {
-    if (!small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, false)) return false;
+    if (!small_graph(g->wtype, g->n, g->m, g->max_w, g->mean_w, 0)) return false;
     if (!p) return true;
     if ((p->flags & ~GBS_F_NO_STATS) || p->solo_entries || p->solo_descs || p->inline_edges || p->full_items ||
         p->fuse_rounds)
@@ -450,12 +461,15 @@ bool small_call(const gbs_graph *g, const gbs_params *p) {
                                   resolve_schedule(g->wtype, g->max_w, g->n, g->m, 0.0, -1.0).delta;
 }
 
-bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, double mean_w, bool batched) {
-    if (n == 0 || n > kSmallN || m > (batched ? kSmallBatchM : kSmallM)) return false;
+bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, double mean_w, uint32_t instances) {
+    if (n == 0 || n > kSmallN || m > (instances ? kSmallBatchM : kSmallM)) return false;
     if (small_shape(n, m).bytes > kSmallBytes) return false;
-    if (!batched && m > kSmallWideM &&
-        resolve_schedule(wt, max_w, n, m, 0.0, -1.0).delta >= kWideRatio * mean_w)
-        return false;
+    if (m > kSmallWideM) {
+        const bool wide = resolve_schedule(wt, max_w, n, m, 0.0, -1.0).delta >= kWideRatio * mean_w;
+        const bool large = m > kSmallM, skewed = max_w > kSkew * mean_w;
+        const uint32_t least = kWideStep * (1u + (large ? 1u : 0u) + (skewed ? 0u : 1u));
+        if ((wide || (large && skewed)) && instances < least) return false;
+    }
     if (wt == GBS_WEIGHT_U32) return (double)n * max_w < 4294967295.0;
     return wt == GBS_WEIGHT_F32;
 }

@@ -17,9 +17,9 @@ SmallShape small_shape(uint32_t n, uint64_t m);
 
 // Whether a graph is solved by one CTA when the caller left every knob of the
 // schedule at its default: uint32 or float32 weights, the size below for its
-// weights (mean_w: their mean), and (for uint32) no path sum that could pass
-// 2^32 - 1.
-bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, double mean_w, bool batched);
+// weights (mean_w: their mean) and, in a plan, the number of instances (0: a
+// call of its own), and (for uint32) no path sum that could pass 2^32 - 1.
+bool small_graph(gbs_weight_type wt, uint32_t n, uint64_t m, double max_w, double mean_w, uint32_t instances);
 
 // Whether this call runs on one CTA: a small graph and no knob set that would
 // shape the run (a delta that resolves to the default width is the default; the

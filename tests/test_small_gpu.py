@@ -156,3 +156,51 @@ def test_small_limit_of_edges(wtype, weights, m, one, gb, orc):
     ref = orc.dijkstra(row, v, w, 3)
     assert (st["blocks"] == 1) == one
     assert np.array_equal(d, ref) and np.array_equal(p, orc.min_tight_pred(row, v, w, 3, ref))
+
+
+@pytest.mark.parametrize("weights,m,one", [
+    ("unit", 131072, {1: True}), ("unit", 131073, {63: False, 64: True}), ("unit", 262145, {64: False}),
+    ("skewed", 131073, {31: False, 32: True}), ("skewed", 262145, {63: False, 64: True}),
+    ("uniform", 524288, {1: True, 2: True})])
+def test_small_plan_limit(weights, m, one, gb, orc):
+    """Instances from which on a plan gives each one CTA (the groups of the other
+    kernel have at least two at these counts)."""
+    n = 8192
+    rng = np.random.default_rng(m)
+    u, v = np.sort(rng.integers(0, n, m)), rng.integers(0, n, m).astype(np.uint32)
+    row = np.zeros(n + 1, dtype=np.uint64)
+    row[1:] = np.cumsum(np.bincount(u, minlength=n))
+    w = {"unit": np.ones(m, np.uint32), "uniform": rng.integers(1, 256, m).astype(np.uint32),
+         "skewed": rng.lognormal(0, 2, m).astype(np.float32)}[weights]
+    with gb.Graph(row, v, w) as g:
+        for k, expect in one.items():
+            src = (np.arange(k, dtype=np.uint32) * 83) % n
+            with gb.Plan(g, src) as plan:
+                st = plan.run()
+                dist, pred = plan.results()
+            assert (st["group_ctas"] == 1) == expect, (k, st)
+            for i in (0, k - 1):
+                ref = orc.dijkstra(row, v, w, int(src[i]))
+                assert np.array_equal(dist[i], ref)
+                assert np.array_equal(pred[i], orc.min_tight_pred(row, v, w, int(src[i]), ref))
+
+
+def test_small_pack_limit(gb, orc):
+    """A pack goes by its number of graphs and every graph's weights."""
+    rng = np.random.default_rng(4)
+    n, m = 4096, 140000
+    u, v = np.sort(rng.integers(0, n, m)), rng.integers(0, n, m).astype(np.uint32)
+    row = np.zeros(n + 1, dtype=np.uint64)
+    row[1:] = np.cumsum(np.bincount(u, minlength=n))
+    wide = gb.HostGraph(row, v, np.ones(m, np.uint32))
+    for graphs, one in (([gb.gen_rmat(8, 8, i) for i in range(40)] + [wide], False),
+                        ([gb.gen_rmat(8, 8, i) for i in range(63)] + [wide], True),
+                        ([gb.HostGraph(row, v, rng.integers(1, 256, m).astype(np.uint32))] * 2, True)):
+        src = np.zeros(len(graphs), np.uint32)
+        with gb.Pack(graphs) as pk, gb.Plan(pk, src) as plan:
+            st = plan.run()
+            dist, _ = plan.results()
+        assert (st["group_ctas"] == 1) == one
+        for i in (0, len(graphs) - 1):
+            h = graphs[i]
+            assert np.array_equal(dist[i], orc.dijkstra(h.row, h.col, h.w, 0))
