@@ -962,16 +962,20 @@ size_t group_bytes(const gbs_graph *g, const BcState *b) {
 // memory.  Beyond L2 a source's big levels fill the GPU alone (R-MAT 22: one).
 uint32_t bc_groups(const gbs_graph *g, const BcState *b, uint32_t want) {
     int l2 = 0;
-    size_t free_b = 0, total_b = 0;
-    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, g->device) != cudaSuccess ||
-        cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    if (want <= 1 || cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, g->device) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }
     const size_t fit = (size_t)l2 / (32 * (size_t)g->n);
+    const uint32_t most = (uint32_t)std::max<size_t>(std::min({(size_t)want, fit, (size_t)b->blocks}), 1);
+    if (most <= std::max(b->groups, 1u)) return most;   // asking for the free memory takes some 20 us
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return 1;
+    }
     const size_t mem = (free_b / 4 + b->groups * group_bytes(g, b)) / group_bytes(g, b);
-    const size_t most = std::min({(size_t)want, fit, mem, (size_t)b->blocks});
-    return (uint32_t)std::max<size_t>(most, 1);
+    return (uint32_t)std::max<size_t>(std::min<size_t>(most, mem), 1);
 }
 
 // Arrays for `groups` sources (kept for later calls; they only grow).
