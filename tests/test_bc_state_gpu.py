@@ -37,3 +37,18 @@ def test_bc_after_cycles_of_tight_edges(wtype, far, single, gb, orc):
             for s in srcs:
                 want = want + (alone if s == 5 else cyc)
             assert np.array_equal(g.betweenness(srcs, **kw)[0], want), srcs
+
+
+@pytest.mark.parametrize("scale", [None, 17])
+def test_bc_of_more_sources_than_groups(scale, gb, orc):
+    """64 sources of one batched launch whose arrays do not fit in L2 together:
+    their passes take several launches, the last of fewer groups."""
+    a = gb.gen_grid(265, 266, 3, "u32", 1, 4) if scale is None else gb.gen_rmat(scale, 2, 3, "u32", 1, 3)
+    assert a.n > 66000
+    srcs = [int(s) for s in gb.sample_sources(a, 65 if scale is None else 40, 7)]
+    with gb.Graph.from_host(a) as g:
+        bc, st = g.betweenness(srcs)
+        again, _ = g.betweenness(srcs[:3])
+    assert st["sources"] == len(srcs)
+    assert np.array_equal(bc, orc.betweenness(a.row, a.col, a.w, srcs))
+    assert np.array_equal(again, orc.betweenness(a.row, a.col, a.w, srcs[:3]))
