@@ -570,6 +570,7 @@ gbs_status launch_run(gbs_graph *g, uint32_t src, const gbs_params *p, void *dis
     a.full_items = (p && p->full_items) ? p->full_items : std::max(g->n, kFullItems);
     a.fuse_rounds = (a.flags & GBS_F_NO_FUSE) ? 0u : ((p && p->fuse_rounds) ? p->fuse_rounds : kFuseRounds);
     merge_limits(g->wtype, g->n, g->m, g->max_deg, g->max_w, learned, a.merge_low, a.merge_ramp, a.merge_drain);
+    a.merge_low = std::min(a.merge_low, a.full_items);   // such a bucket relaxes whole rows
     a.run_ns = a.wait_ns * 16ull;
     a.ctrl = learned ? kCtrlLearned : kCtrlFixed;
     a.span_fixed = 1;

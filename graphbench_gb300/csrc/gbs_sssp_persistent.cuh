@@ -705,6 +705,12 @@ __device__ __forceinline__ void decide_bucket(const SsspArgs &a, Ctl *ctl, const
                 if ((int)lane >= o) incl += y;
             }
             const uint32_t most = a.merge_ramp ? min(kMergeLow, nb / a.merge_ramp + 1u) : kMergeLow;
+            // nor does a drain split a bucket that would not be: the heavy phases
+            // of a grid's buckets cost more than the merge gives (1024^2 grid,
+            // full_items 1024, ms: no merge 40.8, every merge 51.9, none that
+            // splits 31.4)
+            if (a.ctrl == kCtrlFixed && !a.merge_whole && __shfl_sync(FULL, incl, span - 1u) <= a.full_items)
+                wide = min(wide, (uint32_t)__popc(__ballot_sync(FULL, incl <= a.full_items)));
             wide = max(wide, (uint32_t)__popc(__ballot_sync(FULL, lane < most && incl <= a.merge_low)));
         }
         if (wide > span) {

@@ -77,3 +77,18 @@ def test_merges_widen_with_the_distance_on_graphs_that_spread(gb, orc):
                 done += rec["items"]
         assert wide != ramp
         assert np.array_equal(d, orc.dijkstra(r, c, x, 1))
+
+
+@pytest.mark.parametrize("wtype", ["u32", "f32", "f64"])
+def test_no_merge_splits_a_bucket(wtype, gb, orc):
+    """Thin buckets merge up to full_items entries, which relax whole rows: only a
+    drain (of at most four base buckets), and only where the first list alone
+    holds more, merges buckets that are split."""
+    a = gb.gen_grid(300, 320, 4, "f32" if wtype == "f32" else "u32")
+    w = a.w / 3.0 if wtype == "f64" else a.w
+    with gb.Graph(a.row, a.col, w) as g:
+        d, _, _ = g.sssp(1, full_items=700, flags=gb.F_TRACE)
+        starts = _starts(g.trace())
+        assert all(r["full"] and r["items"] <= 700 for r in starts if r["span"] > 4)
+        assert max(r["span"] for r in starts) > 4
+        assert np.array_equal(d, orc.dijkstra(a.row, a.col, w, 1))
