@@ -2,7 +2,7 @@
 //
 // What bounds a small graph is the chain of dependent phases, not its edges:
 // in the persistent kernel a phase of a few hundred entries is a chain of
-// about nine L2 round trips (list, tag, distance, row, edges, target distance,
+// about eight L2 round trips (list, distance, row, edges, target distance,
 // three atomics), 4-10 us, and an R-MAT of 1,024 vertices takes 50 of them.
 // Here the distances, the frontier and the queued sets of the whole graph sit
 // in the shared memory of one CTA, so a sweep is one global round trip (the

@@ -90,9 +90,11 @@ inline uint32_t split_full_items(uint32_t n) { return n / 16u > kFullItems ? n /
 // graph of 1 M vertices and degree 8 (25) 0.88 -> 0.71, 16 (39) 1.17 -> 0.99,
 // lattice with random short links, 1 M (20) 16.8 -> 9.6, 1024^2 grid (4) 28.5
 // -> 10.5, R-MAT 16 (6,299) 0.47 -> 0.35, 18 0.74 -> 0.47, 20 1.05 -> 0.73,
-// 22 (162,304) 1.97 -> 1.60.  A drain of 8 or 16 base buckets gains a little
-// more (R-MAT 20 0.64, 0.61; 22 1.48, 1.43); a learned run, whose base widths
-// the controller picks, takes up to 32.
+// 22 (162,304) 1.97 -> 1.60.  A drain of 8 or 16 base buckets gains 8-16 %
+// more on these (R-MAT 20 0.64, 0.61; 22 1.48, 1.43); it is 4 because the output
+// biases of the committed controller are calibrated against it (learned runs
+// take up to 32 from base widths of their own and are to stay ahead of plain ones
+// on held-out graphs), and no sweep of plans has been made.
 // The ramp (random graphs, ms; no merge in any form, no ramp, a ramp of 4): 64
 // sources of 262,144 vertices and degree 8 (23) 5.10, 6.06, 3.55, degree 4 (16)
 // 3.76, 4.41, 2.48; one source of 1 M vertices and degree 8 1.21, 0.74, 0.66,
@@ -341,8 +343,8 @@ __device__ __forceinline__ bool edge_sum(typename Arith<WT>::D du, typename Arit
 //      is lowered, without waiting for the result, when a vertex that may be
 //      pending is queued elsewhere.  Asking the tag for every target in the
 //      window was a third dependent round trip to L2 per improvement, and
-//      scans read it again: R-MAT of 4 M edges 1505 -> 1397 us of kernel time
-//      without, 64 sources of a 256 k-edge R-MAT 6.13 -> 5.59 ms, 16 of an
+//      scans read it again: R-MAT of 4 M vertices 1505 -> 1397 us of kernel time
+//      without, 64 sources of an R-MAT of 256 k vertices 6.13 -> 5.59 ms, 16 of an
 //      R-MAT 22 23.3 -> 20.9 ms; grids, bound by their chain of phases, the same.
 template <int WT, int U>
 __device__ __forceinline__ void improve_batch(const SsspArgs &a, const Targets &t, const bool (&cand)[U],

@@ -412,9 +412,9 @@ __device__ void rebucket_pending(const SsspArgs &a, const Uniform &U, const Exec
         warp_enqueue<1>(a, t, q, v);
     }
     // the tags just stored and the pending minimum feed the next decision and
-    // the next scan; on one CTA only __syncthreads separates them from this
-    // phase, and it waits neither for the plain stores to reach L2 (where the
-    // scan's L2-only loads read) nor for the reduction
+    // later improvements; on one CTA only __syncthreads separates them from this
+    // phase, and it waits neither for the plain stores to reach L2 (where
+    // atomics and L2-only loads find them) nor for the reduction
     __threadfence();
     // entries that had already left the pending list (statistics / trace)
     for (int o = 16; o > 0; o >>= 1) stale += __shfl_down_sync(0xffffffffu, stale, o);
